@@ -276,17 +276,6 @@ struct LimQueue {
   }
 };
 
-// Arithmetic with explicit rounding: never contracted or reassociated, so an
-// expression written with these gives the same bits wherever it is inlined.
-__device__ __forceinline__ double xadd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double xmul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double xfma(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float xadd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float xmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float xfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double xrcp(double a) { return __drcp_rn(a); }
-__device__ __forceinline__ float xrcp(float a) { return __frcp_rn(a); }
-
 // Characteristic basis of one face, production build: the rows of L = S and
 // R = S^-1 of flux_charteric (OCFD_inviscous_character.f90:216-248) applied
 // without forming the matrices.  AXS: the sweep's metric row has a single
@@ -672,13 +661,16 @@ __device__ __forceinline__ void face_body(const FaceArgs<S>& a, const int bx, co
     const R c = sqrt(T) / ma;  // cc: OCFD_inviscous.f90:67
 #endif
     R fp[5], fm[5];
+#if OCFD_FEWER_DIVS
     if constexpr (AXS) {
       const R Ad = DIR == 0 ? A1 : (DIR == 1 ? A2 : A3);
       if (a.split == 1)
         split_sw_axis<DIR>(ph, gam, c, d, u, v, w, Ad, fp, fm);
       else
         split_llf_axis<DIR>(ph, gam, c, d, u, v, w, Ad, fp, fm);
-    } else {
+    } else
+#endif
+    {
       if (a.split == 1)
         split_sw(ph, gam, c, d, u, v, w, A1, A2, A3, fp, fm);
       else
