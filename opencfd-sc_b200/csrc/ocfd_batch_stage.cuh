@@ -63,11 +63,11 @@ constexpr size_t stage_args_bytes() {
 }
 
 // Dynamic shared memory of the persistent kernel: the largest face tile.
-template <bool CHAR, int V, typename R>
+template <bool CHAR, int SCHEME, int V, typename R>
 constexpr size_t stage_smem() {
-  constexpr size_t a = face_smem<0, CHAR, FaceTileV<0, V>::NP, FaceTileV<0, V>::TF, R>();
-  constexpr size_t b = face_smem<1, CHAR, FaceTileV<1, V>::NP, FaceTileV<1, V>::TF, R>();
-  constexpr size_t c = face_smem<2, CHAR, FaceTileV<2, V>::NP, FaceTileV<2, V>::TF, R>();
+  constexpr size_t a = face_smem<0, CHAR, SCHEME, FaceTileV<0, V>::NP, FaceTileV<0, V>::TF, R>();
+  constexpr size_t b = face_smem<1, CHAR, SCHEME, FaceTileV<1, V>::NP, FaceTileV<1, V>::TF, R>();
+  constexpr size_t c = face_smem<2, CHAR, SCHEME, FaceTileV<2, V>::NP, FaceTileV<2, V>::TF, R>();
   return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
 
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256, OCFD_FACE_MINB) k_batch_stage(StageTab<R>
         case BW_VISC:
           if (VISC) {
             const ViscArgs<R, R>& A = *reinterpret_cast<const ViscArgs<R, R>*>(sa);
-            if (OCFD_VISC_AXS && visc_axis_aligned(A.ph.metzero))
+            if (OCFD_VISC_AXS && metrics_diagonal(A.ph.metzero))
               visc_grad_body<R, R, OCFD_VISC_AXS != 0>(A, bx, by, bz);
             else
               visc_grad_body<R, R>(A, bx, by, bz);
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256, OCFD_FACE_MINB) k_batch_stage(StageTab<R>
 
 template <bool CHAR, int SCHEME, int V, typename R>
 static cudaError_t launch_batch_stage_t(const StageTab<R>& t, int nblocks, cudaStream_t st, int* per_sm) {
-  constexpr size_t smem = stage_smem<CHAR, V, R>();
+  constexpr size_t smem = stage_smem<CHAR, SCHEME, V, R>();
   auto kern = k_batch_stage<CHAR, SCHEME, V, true, R>;
   if (nblocks == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -327,6 +327,15 @@ __host__ __device__ __forceinline__ bool axis_aligned(unsigned int metzero) {
   return (metzero & off) == off;
 }
 
+// Whether every off-diagonal metric the viscous terms read is identically zero
+// (Aky Akz Aix Aiz Asx Asy of the gradients, Aky1 Akz1 Aix1 Aiz1 Asx1 Asy1 of the
+// fluxes): a grid whose axes are the coordinate axes (box, stretched box).
+__host__ __device__ __forceinline__ bool metrics_diagonal(unsigned int metzero) {
+  const unsigned int off = (1u << 4) | (1u << 5) | (1u << 6) | (1u << 8) | (1u << 9) | (1u << 10) | (1u << 14) |
+                           (1u << 15) | (1u << 16) | (1u << 18) | (1u << 19) | (1u << 20);
+  return (metzero & off) == off;
+}
+
 // set_hybrid_scheme: OCFD_SetHybrid.f90:2-15
 __device__ __forceinline__ int hybrid_index(double R0, double t1, double t2) {
   if (R0 <= t1) return 1;

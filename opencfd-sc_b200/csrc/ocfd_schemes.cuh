@@ -11,18 +11,12 @@
 
 #include <cuda_runtime.h>
 
+#include "ocfd_device.cuh"
+
 namespace ocfd {
 
 template <typename R>
 __device__ __forceinline__ R sq(R x) { return x * x; }
-
-#ifndef OCFD_FEWER_DIVS
-#ifdef OCFD_STRICT
-#define OCFD_FEWER_DIVS 0
-#else
-#define OCFD_FEWER_DIVS 1
-#endif
-#endif
 
 // Normalised WENO sum (a0 q0 + ...) / (a0 + ...) with a_k = C_k / (ep + S_k)^2,
 // in the reference's order.  Production FP64 build: every a_k is multiplied by
@@ -217,13 +211,24 @@ __device__ __forceinline__ R weno7M(const R* v) {
   return weno_sum4(ep, C0, C1, C2, C3, S0, S1, S2, S3, q0, q1, q2, q3);
 }
 
-// ---- packed FP32 (production mixed path, sm_100): two reconstructions per
-// instruction.  FFMA2 / FADD2 / FMUL2 apply one IEEE single-precision operation,
-// rounded to nearest, to each of two lanes; the issue-bound FP32 face sweeps
-// issue half the arithmetic instructions.  Lanes round as the scalar operations
-// would, but the contraction into FMAs is fixed here rather than left to the
-// compiler, so results can differ from the scalar form in the last bits; the
-// batched and single-instance sweeps share this code and agree bit for bit.
+// ---- production build: the WENO schemes on differences of the stencil
+// Every candidate, derivative and smoothness indicator of hh_weno7P / hh_weno5P
+// is a combination of the stencil's first, second and third differences, which
+// the candidates share, and the value relative to v(0) is
+//   sum_k w_k (S1_k / 2 + D2_k / 12) / sum_k w_k
+// (WENO7; S1_k the first and D2_k the second derivative of candidate k at the
+// face's left point).  With the mixed term of the indicator completed to a
+// square this is 85 instead of 118 operations a reconstruction in FP64 (the
+// sweeps are bound by the FP64 pipe), and the differences lose no digits to the
+// mean of the fluxes.  hh_weno7M(v) is hh_weno7P of the mirrored window
+// v'(k) = v(1 - k), term for term, so both sides use the same function.
+// All operations are explicitly rounded: single-instance and batched sweeps
+// give the same bits.
+//
+// The arithmetic is written once over a number type: double and float, or F2, two
+// floats per packed instruction (FFMA2 / FADD2 / FMUL2 of sm_100 apply one IEEE
+// single-precision operation to each of two lanes: F+ in lane x, the mirrored F-
+// in lane y, half the instructions for the issue-bound FP32 sweeps).
 #ifndef OCFD_F32X2
 #define OCFD_F32X2 OCFD_FEWER_DIVS
 #endif
@@ -235,51 +240,126 @@ __device__ __forceinline__ F2 f2(float a, float b) { return F2{make_float2(a, b)
 __device__ __forceinline__ F2 add2(F2 a, F2 b) { return F2{__fadd2_rn(a.v, b.v)}; }
 __device__ __forceinline__ F2 mul2(F2 a, F2 b) { return F2{__fmul2_rn(a.v, b.v)}; }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return F2{__ffma2_rn(a.v, b.v, c.v)}; }
+__device__ __forceinline__ F2 xadd(F2 a, F2 b) { return add2(a, b); }
+__device__ __forceinline__ F2 xmul(F2 a, F2 b) { return mul2(a, b); }
+__device__ __forceinline__ F2 xfma(F2 a, F2 b, F2 c) { return fma2(a, b, c); }
+__device__ __forceinline__ F2 xsub(F2 a, F2 b) { return fma2(f2(-1.0f), b, a); }
+__device__ __forceinline__ double xsub(double a, double b) { return __dadd_rn(a, -b); }
+__device__ __forceinline__ float xsub(float a, float b) { return __fadd_rn(a, -b); }
+template <typename T>
+struct Num {
+  static __device__ __forceinline__ T c(double x) { return T(x); }
+};
+template <>
+struct Num<F2> {
+  static __device__ __forceinline__ F2 c(double x) { return f2(float(x)); }
+};
+// reciprocal to within an ulp (FP32 weights)
+__device__ __forceinline__ float fast_rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ F2 fast_rcp(F2 x) { return f2(fast_rcp(x.v.x), fast_rcp(x.v.y)); }
 
-// WENO7 of two windows at once: w[0..6] are the stencil values at offsets -3..3
-// of weno7P.  Lane x: F+ (weno7P of the F+ window); lane y: F- -- weno7M(v) is
-// weno7P of the mirrored window v'(k) = v(1 - k), term for term, so the caller
-// puts F-(1 - k) in lane y of w[k + 3].  Same terms and order as weno7P; the
-// weights' divisions are per lane.
-__device__ __forceinline__ float2 weno7_x2(const F2* w) {
-  const F2 C0 = f2(float(1.0 / 35.0)), C1 = f2(float(12.0 / 35.0)), C2 = f2(float(18.0 / 35.0)), C3 = f2(float(4.0 / 35.0));
-  const F2 m1 = f2(-1.0f), b2 = f2(-2.0f), c3 = f2(3.0f);
-  const F2 *v = w + 3;
-  // S1k, S2k, S3k: weno7P's smoothness differences
-  F2 S10 = fma2(f2(float(11.0 / 6.0)), v[0], fma2(f2(float(-18.0 / 6.0)), v[-1], fma2(f2(float(9.0 / 6.0)), v[-2], mul2(f2(float(-2.0 / 6.0)), v[-3]))));
-  F2 S11 = fma2(f2(float(2.0 / 6.0)), v[1], fma2(f2(float(3.0 / 6.0)), v[0], fma2(m1, v[-1], mul2(f2(float(1.0 / 6.0)), v[-2]))));
-  F2 S12 = fma2(f2(float(-1.0 / 6.0)), v[2], add2(fma2(f2(float(-3.0 / 6.0)), v[0], mul2(f2(float(-2.0 / 6.0)), v[-1])), v[1]));
-  F2 S13 = fma2(f2(float(2.0 / 6.0)), v[3], fma2(f2(float(-9.0 / 6.0)), v[2], fma2(f2(float(18.0 / 6.0)), v[1], mul2(f2(float(-11.0 / 6.0)), v[0]))));
-  F2 S20 = fma2(f2(2.0f), v[0], fma2(f2(-5.0f), v[-1], fma2(f2(4.0f), v[-2], mul2(m1, v[-3]))));
-  F2 S21 = add2(fma2(b2, v[0], v[-1]), v[1]);
-  F2 S22 = add2(fma2(b2, v[1], v[0]), v[2]);
-  F2 S23 = fma2(m1, v[3], fma2(f2(4.0f), v[2], fma2(f2(-5.0f), v[1], mul2(f2(2.0f), v[0]))));
-  F2 S30 = add2(fma2(c3, fma2(m1, v[-1], v[-2]), mul2(m1, v[-3])), v[0]);
-  F2 S31 = add2(fma2(c3, fma2(m1, v[0], v[-1]), mul2(m1, v[-2])), v[1]);
-  F2 S32 = add2(fma2(c3, fma2(m1, v[1], v[0]), mul2(m1, v[-1])), v[2]);
-  F2 S33 = add2(fma2(c3, fma2(m1, v[2], v[1]), mul2(m1, v[0])), v[3]);
-  const F2 d12 = f2(float(13.0 / 12.0)), d13 = f2(float(1043.0 / 960.0)), d14 = f2(float(1.0 / 12.0));
-  auto beta = [&](F2 a, F2 b, F2 c) {
-    return fma2(mul2(d14, a), c, fma2(mul2(d13, c), c, fma2(mul2(d12, b), b, mul2(a, a))));
+// sum_k w_k q_k / (scale sum_k w_k) with w_k = C_k / E_k^2, E_k = ep + S_k.  FP64: every
+// w_k is multiplied by the product of all E_j^2, which leaves the normalised
+// weights unchanged and needs one division (E >= ep, and the indicators of
+// physical fluxes keep the products far inside the double range).  FP32, whose
+// range is too small for the products, takes the reciprocals of the E_k.
+__device__ __forceinline__ double weno_mix4(double C1, double C2, double C3, double E0, double E1, double E2, double E3,
+                                            double q0, double q1, double q2, double q3, double scale) {
+  const double D0 = xmul(E0, E0), D1 = xmul(E1, E1), D2 = xmul(E2, E2), D3 = xmul(E3, E3);
+  const double P01 = xmul(D0, D1), P23 = xmul(D2, D3);
+  const double w0 = xmul(D1, P23), w1 = xmul(xmul(C1, D0), P23), w2 = xmul(xmul(C2, D3), P01),
+               w3 = xmul(xmul(C3, D2), P01);
+  const double num = xfma(w3, q3, xfma(w2, q2, xfma(w1, q1, xmul(w0, q0))));
+  return num / xmul(scale, xadd(xadd(w0, w1), xadd(w2, w3)));
+}
+template <typename T>
+__device__ __forceinline__ T weno_mix4(T C1, T C2, T C3, T E0, T E1, T E2, T E3, T q0, T q1, T q2, T q3, T scale) {
+  const T r0 = fast_rcp(E0), r1 = fast_rcp(E1), r2 = fast_rcp(E2), r3 = fast_rcp(E3);
+  const T w0 = xmul(r0, r0), w1 = xmul(xmul(C1, r1), r1), w2 = xmul(xmul(C2, r2), r2), w3 = xmul(xmul(C3, r3), r3);
+  const T num = xfma(w3, q3, xfma(w2, q2, xfma(w1, q1, xmul(w0, q0))));
+  return xmul(num, fast_rcp(xmul(scale, xadd(xadd(w0, w1), xadd(w2, w3)))));
+}
+__device__ __forceinline__ double weno_mix3(double C0, double C1, double E0, double E1, double E2, double q0, double q1,
+                                            double q2, double scale) {
+  const double D0 = xmul(E0, E0), D1 = xmul(E1, E1), D2 = xmul(E2, E2);
+  const double w0 = xmul(C0, xmul(D1, D2)), w1 = xmul(C1, xmul(D0, D2)), w2 = xmul(D0, D1);
+  const double num = xfma(w2, q2, xfma(w1, q1, xmul(w0, q0)));
+  return num / xmul(scale, xadd(xadd(w0, w1), w2));
+}
+template <typename T>
+__device__ __forceinline__ T weno_mix3(T C0, T C1, T E0, T E1, T E2, T q0, T q1, T q2, T scale) {
+  const T r0 = fast_rcp(E0), r1 = fast_rcp(E1), r2 = fast_rcp(E2);
+  const T w0 = xmul(xmul(C0, r0), r0), w1 = xmul(xmul(C1, r1), r1), w2 = xmul(r2, r2);
+  const T num = xfma(w2, q2, xfma(w1, q1, xmul(w0, q0)));
+  return xmul(num, fast_rcp(xmul(scale, xadd(xadd(w0, w1), w2))));
+}
+
+// hh_weno7P (OCFD_Schemes_1.f90:58-121) minus v(0); e[j] = v(j - 2) - v(j - 3), j = 0..5
+template <typename T>
+__device__ __forceinline__ T weno7_diff(const T* e) {
+  using N = Num<T>;
+  const T a0 = xsub(e[1], e[0]), a1 = xsub(e[2], e[1]), a2 = xsub(e[3], e[2]), a3 = xsub(e[4], e[3]),
+          a4 = xsub(e[5], e[4]);
+  const T t0 = xsub(a1, a0), t1 = xsub(a2, a1), t2 = xsub(a3, a2), t3 = xsub(a4, a3);  // third differences
+  const T half = N::c(0.5), third = N::c(1.0 / 3.0), m6 = N::c(-1.0 / 6.0);
+  const T cen = xmul(half, xadd(e[2], e[3]));
+  const T s0 = xfma(third, t0, xfma(half, a1, e[2])), s1 = xfma(m6, t1, cen), s2 = xfma(m6, t2, cen),
+          s3 = xfma(third, t3, xfma(N::c(-0.5), a3, e[3]));
+  const T b0 = xadd(a1, t0), b3 = xsub(a3, t3);  // second derivatives of the outer candidates
+  // ep + S_k, S = S1^2 + S1 S3 / 12 + 13/12 S2^2 + 1043/960 S3^2; S2 of candidate 2 is the
+  // second difference at v(1), as in the reference
+  auto ind = [&](T d1, T d2, T d3) -> T {
+    const T x = xfma(N::c(1.0 / 24.0), d3, d1);
+    return xfma(xmul(N::c(1043.0 / 960.0 - 1.0 / 576.0), d3), d3,
+                xfma(xmul(N::c(13.0 / 12.0), d2), d2, xfma(x, x, N::c(1.0e-8))));
   };
-  const F2 S0 = beta(S10, S20, S30), S1 = beta(S11, S21, S31), S2 = beta(S12, S22, S32), S3 = beta(S13, S23, S33);
-  // candidate values q0..q3
-  const F2 q0 = fma2(f2(float(25.0 / 12.0)), v[0], fma2(f2(float(-23.0 / 12.0)), v[-1], fma2(f2(float(13.0 / 12.0)), v[-2], mul2(f2(float(-3.0 / 12.0)), v[-3]))));
-  const F2 q1 = fma2(f2(float(3.0 / 12.0)), v[1], fma2(f2(float(13.0 / 12.0)), v[0], fma2(f2(float(-5.0 / 12.0)), v[-1], mul2(f2(float(1.0 / 12.0)), v[-2]))));
-  const F2 q2 = fma2(f2(float(-1.0 / 12.0)), v[2], fma2(f2(float(7.0 / 12.0)), v[1], fma2(f2(float(7.0 / 12.0)), v[0], mul2(f2(float(-1.0 / 12.0)), v[-1]))));
-  const F2 q3 = fma2(f2(float(1.0 / 12.0)), v[3], fma2(f2(float(-5.0 / 12.0)), v[2], fma2(f2(float(13.0 / 12.0)), v[1], mul2(f2(float(3.0 / 12.0)), v[0]))));
-  // weights a_k = C_k / (ep + S_k)^2 (divisions per lane), normalised sum
-  const F2 ep = f2(float(1.0e-8));
-  F2 D0 = add2(ep, S0), D1 = add2(ep, S1), D2 = add2(ep, S2), D3 = add2(ep, S3);
-  D0 = mul2(D0, D0);
-  D1 = mul2(D1, D1);
-  D2 = mul2(D2, D2);
-  D3 = mul2(D3, D3);
-  const F2 a0 = f2(C0.v.x / D0.v.x, C0.v.y / D0.v.y), a1 = f2(C1.v.x / D1.v.x, C1.v.y / D1.v.y);
-  const F2 a2 = f2(C2.v.x / D2.v.x, C2.v.y / D2.v.y), a3 = f2(C3.v.x / D3.v.x, C3.v.y / D3.v.y);
-  const F2 am = add2(add2(add2(a0, a1), a2), a3);
-  const F2 num = fma2(a3, q3, fma2(a2, q2, fma2(a1, q1, mul2(a0, q0))));
-  return make_float2(num.v.x / am.v.x, num.v.y / am.v.y);
+  const T six = N::c(6.0);
+  return weno_mix4(N::c(12.0), N::c(18.0), N::c(4.0), ind(s0, b0, t0), ind(s1, a2, t1), ind(s2, a3, t2),
+                   ind(s3, b3, t3), xfma(six, s0, b0), xfma(six, s1, a2), xfma(six, s2, a2), xfma(six, s3, b3),
+                   N::c(12.0));
+}
+// hh_weno5P (OCFD_Schemes_1.f90:9-29) minus v(0); e as above (e[1..4] are read)
+template <typename T>
+__device__ __forceinline__ T weno5_diff(const T* e) {
+  using N = Num<T>;
+  auto ind = [&](T d1, T d2) -> T {
+    return xfma(xmul(N::c(0.25), d1), d1, xfma(xmul(N::c(13.0 / 12.0), d2), d2, N::c(1.0e-6)));
+  };
+  const T E0 = ind(xfma(N::c(-3.0), e[3], e[4]), xsub(e[4], e[3])), E1 = ind(xadd(e[2], e[3]), xsub(e[3], e[2])),
+          E2 = ind(xfma(N::c(-3.0), e[2], e[1]), xsub(e[2], e[1]));
+  // candidates times 6
+  const T q0 = xfma(N::c(4.0), e[3], xmul(N::c(-1.0), e[4])), q1 = xfma(N::c(2.0), e[3], e[2]),
+          q2 = xfma(N::c(5.0), e[2], xmul(N::c(-2.0), e[1]));
+  return weno_mix3(N::c(3.0), N::c(6.0), E0, E1, E2, q0, q1, q2, N::c(6.0));
+}
+template <int SCHEME, typename T>
+__device__ __forceinline__ T weno_diff(const T* e) {
+  if (SCHEME == 1) return weno5_diff(e);
+  return weno7_diff(e);
+}
+// Sum of both sides' WENO values relative to their upwind points.  vp[k] = F+(k - 3),
+// vm[k] = F-(4 - k) (mirrored), k = 0..6; FP32: the sides in the two lanes.
+template <int SCHEME>
+__device__ __forceinline__ double weno_pair(const double* vp, const double* vm) {
+  double e[6];
+#pragma unroll
+  for (int k = 0; k < 6; k++) e[k] = xsub(vp[k + 1], vp[k]);
+  const double hp = weno_diff<SCHEME>(e);
+#pragma unroll
+  for (int k = 0; k < 6; k++) e[k] = xsub(vm[k + 1], vm[k]);
+  return xadd(hp, weno_diff<SCHEME>(e));
+}
+template <int SCHEME>
+__device__ __forceinline__ float weno_pair(const float* vp, const float* vm) {
+  F2 e[6];
+#pragma unroll
+  for (int k = 0; k < 6; k++) e[k] = xsub(f2(vp[k + 1], vm[k + 1]), f2(vp[k], vm[k]));
+  const F2 h = weno_diff<SCHEME>(e);
+  return xadd(h.v.x, h.v.y);
 }
 
 // minmod2 / minmod4: OCFD_Schemes.f90:274-289

@@ -19,11 +19,13 @@ namespace ocfd {
 
 // Tile geometry of one face sweep (NP pencils x TF faces, stencil TF + 7 points).
 // A = elements per 16 bytes.  x is the innermost (i) dimension of the haloed array.
-template <int DIR, int NP, int TF, typename S>
+// FPT: faces per thread; with two, phase 1 of the x sweep reads a tile across its
+// rows, and two more elements a row keep those reads free of bank conflicts.
+template <int DIR, int NP, int TF, typename S, int FPT = 1>
 struct TmaBox {
   static constexpr int A = 16 / (int)sizeof(S);
   static constexpr int rup(int x) { return (x + A - 1) / A * A; }
-  static constexpr int BX = DIR == 0 ? rup(TF + 7 + A - 1) : rup(NP + A - 1);
+  static constexpr int BX = DIR == 0 ? rup(TF + 7 + A - 1) + (FPT > 1 ? A : 0) : rup(NP + A - 1);
   static constexpr int BY = DIR == 0 ? NP : (DIR == 1 ? TF + 7 : 1);
   static constexpr int BZ = DIR == 2 ? TF + 7 : 1;
   static constexpr int ELEMS = BX * BY * BZ;

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256, OCFD_VISCB_MINB) k_visc_grad_batch(BatchT
   const int q = batch_locate(b, blockIdx.x, bx, by, bz);
   const ViscArgs<R, S>& A = batch_args(b, q, &sa);
   // the member's own variant, as its single-instance launch chooses it
-  if (OCFD_VISC_AXS && visc_axis_aligned(A.ph.metzero))
+  if (OCFD_VISC_AXS && metrics_diagonal(A.ph.metzero))
     visc_grad_body<R, S, OCFD_VISC_AXS != 0>(A, bx, by, bz);
   else
     visc_grad_body<R, S>(A, bx, by, bz);
@@ -76,7 +76,7 @@ template <typename R, typename S>
 cudaError_t launch_visc_grad(const ViscArgs<R, S>& a, cudaStream_t st) {
   const SlabOrder so = slab_order(a.g);
   constexpr bool kAx = OCFD_VISC_AXS != 0;
-  const bool ax = kAx && visc_axis_aligned(a.ph.metzero);
+  const bool ax = kAx && metrics_diagonal(a.ph.metzero);
   if (so.sy == so.gy) {
     if (ax)
       k_visc_grad<R, S, false, kAx><<<update_dims(a.g), 256, 0, st>>>(a, so);

@@ -152,27 +152,19 @@ __device__ __forceinline__ V d0(F at, int l, int nn, int periodic, int cd8, D0C<
 // ---------------------------------------------------------------------------
 // du_viscous part 1 (OCFD_viscous.f90:193-264): comput_Amu (:135-149), the 12
 // gradients, stress and heat flux, and the contravariant viscous fluxes Ev.
-// Whether every off-diagonal metric the viscous body reads is identically zero
-// (Aky Akz Aix Aiz Asx Asy of the gradients, Aky1 Akz1 Aix1 Aiz1 Asx1 Asy1 of the
-// fluxes): a grid whose axes are the coordinate axes (box, stretched box).
 #ifndef OCFD_VISC_AXS
 #define OCFD_VISC_AXS OCFD_FEWER_DIVS
 #endif
-__host__ __device__ __forceinline__ bool visc_axis_aligned(unsigned int metzero) {
-  const unsigned int off = (1u << 4) | (1u << 5) | (1u << 6) | (1u << 8) | (1u << 9) | (1u << 10) | (1u << 14) |
-                           (1u << 15) | (1u << 16) | (1u << 18) | (1u << 19) | (1u << 20);
-  return (metzero & off) == off;
-}
-
-// AXS (production build, visc_axis_aligned grids): the Cartesian gradients and
+// AXS (production build, metrics_diagonal grids): the Cartesian gradients and
 // the contravariant fluxes take only the diagonal metrics -- the general form's
 // other terms add exact zeros, so the values are the same (up to the sign of a
 // zero) with a third of the metric registers and products.
-template <typename R, typename S, bool AXS = false>
+// A block covers 32 x ROWS points of plane bz (32 * ROWS threads).
+template <typename R, typename S, bool AXS = false, int ROWS = 8>
 __device__ __forceinline__ void visc_grad_body(const ViscArgs<R, S>& a, const int bx, const int by, const int bz) {
   const Grid& G = a.g;
   const int i = bx * 32 + (threadIdx.x & 31) + 1;
-  const int j = by * 8 + (threadIdx.x >> 5) + 1;
+  const int j = by * ROWS + (threadIdx.x >> 5) + 1;
   const int k = bz + 1;
   if (i > G.nx || j > G.ny) return;
   const long long c = G.ih(i, j, k);
