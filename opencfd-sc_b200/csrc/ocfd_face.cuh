@@ -10,10 +10,11 @@
 // (:162-416) for the characteristic form.
 //
 // Tiling: a block owns NP pencils x TF consecutive faces along the sweep
-// direction (NP*TF = 256 threads, one face per thread).  Phase 1 loads the
+// direction (128 or 256 faces, one or two per thread).  Phase 1 loads the
 // TF+7 points of its stencil (coalesced along i for x, across i for y/z),
 // computes the split fluxes once per point and stages them in shared memory.
-// Phase 2 computes one face per thread from a register window of 8 points.
+// Phase 2 computes the faces from their windows of 8 points; the uncommon ones
+// (hybrid WENO, OMP6 limiter, boundary closure) go through lists of the block.
 // For a periodic direction face 0 equals face n bit for bit, so only faces
 // 1..n are computed: n faces for n points, no tile does extra work.
 #pragma once
@@ -24,19 +25,15 @@
 #include "ocfd_schemes.cuh"
 #include "ocfd_tma.cuh"
 
-#ifndef OCFD_FPT
-#define OCFD_FPT 1
-#endif
-
 namespace ocfd {
 
 // Tile shapes (NP pencils x TF faces, one face per thread).  Variants 0 and 1
 // (256 threads) are the choices of the batch autotuner -- variant 1 (TF = 32)
 // wastes fewer threads on short pencils.  Variant 2 (128 threads) is the
-// single-instance tile of the characteristic OMP6 sweeps: at 256^3 it measured
-// 5-9% faster there than variant 0 (four blocks per SM overlap one another's
-// barrier and load phases better than two), but slower on the hybrid and
-// WENO7 sweeps, which keep variant 0.  Variants 3 (64 threads) and 4 (128
+// single-instance tile of the characteristic OMP6 and the hybrid sweeps: at 256^3
+// it measured 5-9% faster with OMP6 than variant 0 (four blocks per SM overlap one
+// another's barrier and load phases better than two), but slower on the WENO7
+// sweeps, which keep variant 0.  Variants 3 (64 threads) and 4 (128
 // threads, TF = 32 along y and z) measured slower.
 template <int DIR, int V>
 struct FaceTileV;
@@ -102,13 +99,13 @@ struct FaceTileV<2, 4> {
 // directions.  Their common face is the linear scheme, 80 multiply-adds on 80 values
 // read from shared memory, and two neighbouring faces share seven of their eight
 // points; the longer tile also recomputes 7 halo points for 32 faces instead of 16
-// (isotropic turbulence 320^3, LLF: the three sweeps 11.7 -> 9.5 ms per step).  The
+// (isotropic turbulence 320^3, LLF: the three sweeps 11.4 -> 9.2 ms per step).  The
 // characteristic OMP6 sweeps, with five times the arithmetic per value read, lost
-// more to the halved number of threads (8.1 -> 8.3 ms at 256^3).
+// more to the halved number of threads (a step at 256^3 14.12 -> 14.31 ms).
 template <int DIR, bool CHAR, int SCHEME, typename R, bool ALLIN>
 struct FaceTile {
   static constexpr bool HYB = OCFD_FEWER_DIVS && SCHEME == SCH_HYBRID;
-  static constexpr int FPT = (HYB && ALLIN && sizeof(R) == 8) ? OCFD_FPT : 1;
+  static constexpr int FPT = (HYB && ALLIN && sizeof(R) == 8) ? 2 : 1;
   using V = FaceTileV<DIR, ((CHAR && SCHEME == SCH_OMP6) || HYB) ? 2 : 0>;
   static constexpr int NP = FPT > 1 ? 8 : V::NP, TF = FPT > 1 ? 32 : V::TF, NT = NP * TF / FPT;
 };
