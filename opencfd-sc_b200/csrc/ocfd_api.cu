@@ -410,6 +410,8 @@ int ocfd_gpu_create(const ocfd_params* pin, int device, ocfd_handle** out) {
   if (e != cudaSuccess) return bad(e, "cudaStreamCreate");
   e = setup_face_kernels();
   if (e != cudaSuccess) return bad(e, "setup_face_kernels");
+  e = setup_phase_kernels();
+  if (e != cudaSuccess) return bad(e, "setup_phase_kernels");
   const Grid& g = h->g;
   const size_t n = (size_t)g.n, nh = (size_t)g.nh;
   const size_t r = h->mixed ? 4 : 8;
@@ -851,6 +853,13 @@ static ViscArgs<R, S> visc_args(ocfd_handle* h) {
   return a;
 }
 
+template <typename R>
+static int phase(ocfd_handle* h) {
+  FaceArgs<R> f[3] = {face_args<R>(h, 0), face_args<R>(h, 1), face_args<R>(h, 2)};
+  CK((launch_phase<R>(h->chr, h->p.scheme_invis, f, visc_args<R, R>(h), h->st)));
+  return OCFD_OK;
+}
+
 template <typename R, typename S>
 static int visc_grad(ocfd_handle* h) {
   CK((launch_visc_grad<R, S>(visc_args<R, S>(h), h->st)));
@@ -1024,6 +1033,19 @@ static void prof_mark(ocfd_handle* h, Prof* pf, int group) {
   cudaEventRecord(pf->ev[pf->n++], h->st);
 }
 
+// The sweeps and the viscous gradients of a small grid go out as one launch
+// (ocfd_phase.cuh).  The line, 1 MiB an array (50^3 points in FP64, 64^3 in FP32), lies
+// where a sweep stops being about one wave of blocks, so that its launch gap and idle
+// SMs are most of its time.  Four launches against one, ms per step: WENO7 32^3 mixed
+// 0.064 / 0.047, FP64 0.092 / 0.069; hybrid 48^3 FP64 0.200 / 0.151; 64^3 mixed WENO7
+// 0.176 / 0.161, OMP6 0.213 / 0.186.  Past it the roles share one register and
+// shared-memory limit for nothing: 64^3 FP64 OMP6 0.326 / 0.348, 96^3 WENO7 0.951 /
+// 0.987, mixed 0.508 / 0.518, 256^3 OMP6 14.1 / 16.7.
+constexpr long long PHASE_MAX_BYTES = 1LL << 20;
+static bool phase_merged(const ocfd_handle* h) {
+  return h->p.if_viscous && phase_supported(h->ph) && h->g.n * (h->mixed ? 4 : 8) <= PHASE_MAX_BYTES;
+}
+
 // One RK stage of NS_solver (OCFD_NS_Solver.f90:35-58) on the fused path.
 // Timing groups: 0 sensor, 1-3 face x/y/z, 4 viscous gradients, 5 stage tail,
 // 6 negative-T repair + BC + halos.
@@ -1033,15 +1055,18 @@ static int fused_stage(ocfd_handle* h, int krk, Prof* pf = nullptr) {
     int r = ocfd_gpu_rhybrid(h);
     if (r) return r;
   }
-  const Grid& g = h->g;
-  for (int d = 0; d < 3; d++) {
+  const bool merged = !pf && phase_merged(h);
+  if (merged) {
+    int r = h->mixed ? phase<float>(h) : phase<double>(h);
+    if (r) return r;
+  }
+  for (int d = 0; !merged && d < 3; d++) {
     prof_mark(h, pf, 1 + d);
     int r = h->mixed ? faces<float, float>(h, d) : faces<double, double>(h, d);
     if (r) return r;
   }
-  (void)g;
   prof_mark(h, pf, 4);
-  if (h->p.if_viscous) {
+  if (!merged && h->p.if_viscous) {
     int r = h->mixed ? visc_grad<float, float>(h) : visc_grad<double, double>(h);
     if (r) return r;
   }

@@ -162,6 +162,17 @@ cudaError_t setup_face_batch_kernels_f32();
 template <typename R, typename S>
 cudaError_t launch_visc_grad(const ViscArgs<R, S>& a, cudaStream_t st);
 
+// The three face sweeps and the viscous gradients in one launch (ocfd_phase.cuh):
+// production build, periodic in the three directions, axis-aligned metrics.  An
+// empty grid (v.g.n == 0) sets the kernels' shared-memory limits instead.
+template <typename R>
+cudaError_t launch_phase(bool chr, int scheme, const FaceArgs<R> f[3], const ViscArgs<R, R>& v, cudaStream_t st);
+cudaError_t setup_phase_kernels();
+inline bool phase_supported(const Phys& ph) {
+  return OCFD_FEWER_DIVS && ph.periodic[0] && ph.periodic[1] && ph.periodic[2] && axis_aligned<0>(ph.metzero) &&
+         axis_aligned<1>(ph.metzero) && axis_aligned<2>(ph.metzero) && metrics_diagonal(ph.metzero);
+}
+
 // du = inviscous flux divergence (+ mass force)
 template <typename R>
 cudaError_t launch_div_inv(const UpdArgs<R>& a, cudaStream_t st);
