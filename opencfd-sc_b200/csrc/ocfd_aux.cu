@@ -71,6 +71,21 @@ __device__ __forceinline__ void decode(const Grid& G, long long t, int& i, int& 
   k = (int)(t / ((long long)G.nx * G.ny)) + 1;
 }
 
+// f(i, j, k) at every interior point: the blocks stride over 32 x 8 tiles of the
+// planes (256 threads), so that a point's indices cost no division; decoding a
+// linear index takes three 64-bit ones, which were half of the time of the
+// diagnostics (192^3: ana_box, Q and show_flow_msg, with the download of Q, 2.38 -> 1.92 ms).
+template <typename F>
+__device__ __forceinline__ void for_points(const Grid& G, F f) {
+  const int gx = (G.nx + 31) / 32, gy = (G.ny + 7) / 8, tiles = gx * gy * G.nz;
+  const int di = threadIdx.x & 31, dj = threadIdx.x >> 5;
+  for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
+    const int r = b / gx, k = r / gy;
+    const int i = (b - r * gx) * 32 + di + 1, j = (r - k * gy) * 8 + dj + 1;
+    if (i <= G.nx && j <= G.ny) f(i, j, k + 1);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // comput_Rhybrid (OCFD_SetHybrid.f90:17-152)
 struct Patches {
@@ -575,16 +590,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_flow_msg(Grid G, Phys ph, const
   const double p00 = 1.0 / (ph.gamma * ph.ma * ph.ma);
   const double tmp1 = 1.0 - ph.gamma;
   double s[3] = {0.0, 0.0, 0.0};
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < G.n; t += (long long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    decode(G, t, i, j, k);
+  for_points(G, [&](int i, int j, int k) {
     const long long c = G.ih(i, j, k);
     const double tmp0 = 1.0 / ajac[c];
     const double dd = d[c], uu = u[c], vv = v[c], ww = w[c];
-    s[0] += f[t + 4 * G.n] * tmp0;
+    s[0] += f[G.ii(i, j, k) + 4 * G.n] * tmp0;
     s[1] += dd * (uu * uu + vv * vv + ww * ww) * 0.5 * tmp0;
     s[2] += p00 * pow(dd, tmp1) * T[c] * tmp0;
-  }
+  });
   block_sum<3>(s, sm);
   if (threadIdx.x == 0)
     for (int q = 0; q < 3; q++) part[blockIdx.x * 3 + q] = s[q];
@@ -598,27 +611,29 @@ cudaError_t launch_flow_msg(const Grid& g, const Phys& ph, const double* f, doub
 }
 
 // ana_box sums (OCFD_ANA.f90:209-247) and the d_rms pass (:277-287)
-__global__ void __launch_bounds__(RED_THREADS) k_ana_box(Grid G, Phys ph, DCoef dc, const double* d, const double* u,
+// (three blocks per SM: the fourteen sums and nine gradients take 85 registers)
+constexpr int BOX_BLOCKS = 148 * 3;
+__global__ void __launch_bounds__(RED_THREADS, 3) k_ana_box(Grid G, Phys ph, DCoef dc, const double* d, const double* u,
                                                          const double* v, const double* w, const double* T,
                                                          MetPtrs mp, double* part) {
   __shared__ double sm[14 * RED_THREADS];
   double s[14];
   for (int q = 0; q < 14; q++) s[q] = 0.0;
   const int cd8 = ph.scheme_vis == 6;
-  double* const* M = mp.m;
+  auto M = [&](int m, long long c) -> double { return met_at<double>(ph, m, mp.m[m], c); };
   const double Tsb = 110.4 / ph.ref_amu_t0, TmpR = 1.0 / ph.re;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < G.n; t += (long long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    decode(G, t, i, j, k);
+  for_points(G, [&](int i, int j, int k) {
     const long long c = G.ih(i, j, k);
     const long long st[3] = {1, (long long)G.nxh, (long long)G.nxh * G.nyh};
     const int l[3] = {i, j, k};
     const double* q3[3] = {u, v, w};
     double gr[3][3];
+#pragma unroll
     for (int q = 0; q < 3; q++)
+#pragma unroll
       for (int dd = 0; dd < 3; dd++) gr[q][dd] = d0h(q3[q] + c, st[dd], l[dd], G.len(dd), ph.periodic[dd], cd8, dc, dd);
-    const double Akx = M[3][c], Aky = M[4][c], Akz = M[5][c], Aix = M[6][c], Aiy = M[7][c], Aiz = M[8][c];
-    const double Asx = M[9][c], Asy = M[10][c], Asz = M[11][c];
+    const double Akx = M(3, c), Aky = M(4, c), Akz = M(5, c), Aix = M(6, c), Aiy = M(7, c), Aiz = M(8, c);
+    const double Asx = M(9, c), Asy = M(10, c), Asz = M(11, c);
     const double ux = gr[0][0] * Akx + gr[0][1] * Aix + gr[0][2] * Asx;
     const double uy = gr[0][0] * Aky + gr[0][1] * Aiy + gr[0][2] * Asy;
     const double uz = gr[0][0] * Akz + gr[0][1] * Aiz + gr[0][2] * Asz;
@@ -644,7 +659,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_ana_box(Grid G, Phys ph, DCoef 
     s[11] += uu * uu * uu;
     s[12] += (uu * uu) * (uu * uu);
     s[13] += (wy - vz) * (wy - vz) + (uz - wx) * (uz - wx) + (vx - uy) * (vx - uy);
-  }
+  });
   block_sum<14>(s, sm);
   if (threadIdx.x == 0)
     for (int q = 0; q < 14; q++) part[blockIdx.x * 14 + q] = s[q];
@@ -653,12 +668,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_drms(Grid G, const double* d, c
   __shared__ double sm[RED_THREADS];
   const double d_aver = sums[6] / (double)(G.nx * G.ny * G.nz);
   double s[1] = {0.0};
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < G.n; t += (long long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    decode(G, t, i, j, k);
+  for_points(G, [&](int i, int j, int k) {
     const double x = d[G.ih(i, j, k)] - d_aver;
     s[0] += x * x;
-  }
+  });
   block_sum<1>(s, sm);
   if (threadIdx.x == 0) part[blockIdx.x] = s[0];
 }
@@ -668,8 +681,8 @@ cudaError_t launch_ana_box(const Grid& g, const Phys& ph, const DCoef& dc, doubl
                            cudaStream_t st) {
   MetPtrs mp;
   for (int m = 0; m < 22; m++) mp.m[m] = const_cast<double*>(met[m]);
-  k_ana_box<<<RED_BLOCKS, RED_THREADS, 0, st>>>(g, ph, dc, prim[0], prim[1], prim[2], prim[3], prim[4], mp, scratch);
-  k_final_sum<14><<<1, RED_THREADS, 0, st>>>(scratch, RED_BLOCKS, out14);
+  k_ana_box<<<BOX_BLOCKS, RED_THREADS, 0, st>>>(g, ph, dc, prim[0], prim[1], prim[2], prim[3], prim[4], mp, scratch);
+  k_final_sum<14><<<1, RED_THREADS, 0, st>>>(scratch, BOX_BLOCKS, out14);
   k_drms<<<RED_BLOCKS, RED_THREADS, 0, st>>>(g, prim[0], out14, scratch);
   k_final_sum<1><<<1, RED_THREADS, 0, st>>>(scratch, RED_BLOCKS, out_drms);
   return cudaGetLastError();
@@ -680,22 +693,26 @@ cudaError_t launch_ana_box(const Grid& g, const Phys& ph, const DCoef& dc, doubl
 
 // ana_getQ (OCFD_ANA.f90:127-171): Q = II(grad u) from the CD6/CD8 derivatives of
 // u, v, w (halos exchanged by the caller) and the metrics.
-__global__ void k_ana_q(Grid G, Phys ph, DCoef dc, const double* u, const double* v, const double* w, MetPtrs mp,
-                        double* q) {
+__global__ void __launch_bounds__(256) k_ana_q(Grid G, Phys ph, DCoef dc, const double* u, const double* v,
+                                               const double* w, MetPtrs mp, double* q) {
   const int cd8 = ph.scheme_vis == 6;
-  double* const* M = mp.m;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < G.n; t += (long long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    decode(G, t, i, j, k);
+  auto M = [&](int m, long long c) -> double { return met_at<double>(ph, m, mp.m[m], c); };
+  {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31) + 1;
+    const int j = blockIdx.y * 8 + (threadIdx.x >> 5) + 1;
+    const int k = blockIdx.z + 1;
+    if (i > G.nx || j > G.ny) return;
     const long long c = G.ih(i, j, k);
     const long long st[3] = {1, (long long)G.nxh, (long long)G.nxh * G.nyh};
     const int l[3] = {i, j, k};
     const double* q3[3] = {u, v, w};
     double gr[3][3];
+#pragma unroll
     for (int a = 0; a < 3; a++)
+#pragma unroll
       for (int dd = 0; dd < 3; dd++) gr[a][dd] = d0h(q3[a] + c, st[dd], l[dd], G.len(dd), ph.periodic[dd], cd8, dc, dd);
-    const double Akx = M[3][c], Aky = M[4][c], Akz = M[5][c], Aix = M[6][c], Aiy = M[7][c], Aiz = M[8][c];
-    const double Asx = M[9][c], Asy = M[10][c], Asz = M[11][c];
+    const double Akx = M(3, c), Aky = M(4, c), Akz = M(5, c), Aix = M(6, c), Aiy = M(7, c), Aiz = M(8, c);
+    const double Asx = M(9, c), Asy = M(10, c), Asz = M(11, c);
     const double ux = gr[0][0] * Akx + gr[0][1] * Aix + gr[0][2] * Asx;
     const double vx = gr[1][0] * Akx + gr[1][1] * Aix + gr[1][2] * Asx;
     const double wx = gr[2][0] * Akx + gr[2][1] * Aix + gr[2][2] * Asx;
@@ -705,14 +722,14 @@ __global__ void k_ana_q(Grid G, Phys ph, DCoef dc, const double* u, const double
     const double uz = gr[0][0] * Akz + gr[0][1] * Aiz + gr[0][2] * Asz;
     const double vz = gr[1][0] * Akz + gr[1][1] * Aiz + gr[1][2] * Asz;
     const double wz = gr[2][0] * Akz + gr[2][1] * Aiz + gr[2][2] * Asz;
-    q[t] = ux * vy + ux * wz + vy * wz - uy * vx - uz * wx - vz * wy;
+    q[G.ii(i, j, k)] = ux * vy + ux * wz + vy * wz - uy * vx - uz * wx - vz * wy;
   }
 }
 cudaError_t launch_ana_q(const Grid& g, const Phys& ph, const DCoef& dc, double* const prim[5],
                          const double* const met[22], double* q, cudaStream_t st) {
   MetPtrs mp;
   for (int m = 0; m < 22; m++) mp.m[m] = const_cast<double*>(met[m]);
-  k_ana_q<<<148 * 8, 256, 0, st>>>(g, ph, dc, prim[1], prim[2], prim[3], mp, q);
+  k_ana_q<<<update_dims(g), 256, 0, st>>>(g, ph, dc, prim[1], prim[2], prim[3], mp, q);
   return cudaGetLastError();
 }
 
@@ -721,12 +738,11 @@ cudaError_t launch_ana_q(const Grid& g, const Phys& ph, const DCoef& dc, double*
 __global__ void k_ana_average(Grid G, const double* d, const double* u, const double* v, const double* w,
                               const double* T, double* mean, double K) {
   const double* Q[5] = {d, u, v, w, T};
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < G.n; t += (long long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    decode(G, t, i, j, k);
-    const long long c = G.ih(i, j, k);
+  for_points(G, [&](int i, int j, int k) {
+    const long long c = G.ih(i, j, k), t = G.ii(i, j, k);
+#pragma unroll
     for (int a = 0; a < 5; a++) mean[t + a * G.n] = (K * mean[t + a * G.n] + Q[a][c]) / (K + 1.0);
-  }
+  });
 }
 cudaError_t launch_ana_average(const Grid& g, double* const prim[5], double* mean, int K, cudaStream_t st) {
   k_ana_average<<<148 * 8, 256, 0, st>>>(g, prim[0], prim[1], prim[2], prim[3], prim[4], mean, (double)K);
