@@ -673,17 +673,14 @@ static int halo_all(ocfd_handle* h) {
   PtrList<double> L;
   L.n = 5;
   for (int q = 0; q < 5; q++) L.p[q] = h->prim[q];
-  CK(launch_halo(h->g, h->ph.periodic, L, h->st));
+  PtrList<float> L32{};
+  PtrList<float4> L4{};
   if (h->mixed) {
-    PtrList<float> L32;
-    L32.n = 1;
+    L32.n = L4.n = 1;
     L32.p[0] = h->p32[0];
-    CK(launch_halo_f32(h->g, h->ph.periodic, L32, h->st));
-    PtrList<float4> L4;
-    L4.n = 1;
     L4.p[0] = reinterpret_cast<float4*>(h->q32);
-    CK(launch_halo_f32x4(h->g, h->ph.periodic, L4, h->st));
   }
+  CK(launch_halo(h->g, h->ph.periodic, L, h->st, L32, L4));
   return OCFD_OK;
 }
 

@@ -200,9 +200,8 @@ cudaError_t launch_negt_fix_batch(const BatchTab<UpdArgs<double>>& b, cudaStream
 inline dim3 update_dims(const Grid& g) { return dim3((g.nx + 31) / 32, (g.ny + 7) / 8, g.nz); }
 
 // periodic face halo of narr haloed arrays (exchange_boundary_xyz)
-cudaError_t launch_halo(const Grid& g, const int periodic[3], PtrList<double> arrs, cudaStream_t st);
-cudaError_t launch_halo_f32x4(const Grid& g, const int periodic[3], PtrList<float4> arrs, cudaStream_t st);
-cudaError_t launch_halo_f32(const Grid& g, const int periodic[3], PtrList<float> arrs, cudaStream_t st);
+cudaError_t launch_halo(const Grid& g, const int periodic[3], PtrList<double> a64, cudaStream_t st,
+                        PtrList<float> a32 = {}, PtrList<float4> a128 = {});
 // BC dispatch on the primitives (blunt2d / user isothermal wall)
 cudaError_t launch_bc_wall(const Grid& g, const Phys& ph, double* const prim[5], cudaStream_t st);
 // BC_BoundaryLayer / BC_SweptCorner (OCFD_BC_Boundarylayers.f90): boundary data
