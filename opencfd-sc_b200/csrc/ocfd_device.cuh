@@ -65,6 +65,7 @@ struct Phys {
   double inv_2g;    // 1/(2 gamma)
   double inv_g;     // 1/gamma
   double inv_gm1;   // 1/(gamma-1)
+  double sw_tmp3;   // (3-gamma)/(2(gamma-1))
   double inv_cv;    // 1/Cv
   // bit m: metric array m is +0.0 wherever the kernels read it (box grids:
   // the off-diagonal metrics); its loads are skipped
@@ -257,22 +258,41 @@ __device__ __forceinline__ void split_llf_axis(const Phys& ph, R g, R c, R d, R 
   split_llf_from(ph, c, d, u, v, w, DIR == 0 ? A : R(0), DIR == 1 ? A : R(0), DIR == 2 ? A : R(0),
                  xmul(A, DIR == 0 ? u : (DIR == 1 ? v : w)), xmul(fabs(A), c), fp, fm);
 }
-#else
+#endif
+
+// The splittings in the reference's operations: the strict build, and in the
+// production build (which takes its reciprocals from Phys) the mixed-precision
+// hybrid sweeps (face_on_values in ocfd_face.cuh).
+//
 // Steger-Warming splitting of one point: split_Stager_Warming,
 // OCFD_flux_split.f90:5-70 (the P2 term is dropped there, :51-60).
 template <typename R>
-__device__ __forceinline__ void split_sw(const Phys& ph, R g, R c, R d, R u, R v, R w, R A1, R A2, R A3, R* fp,
-                                         R* fm) {
+__device__ __forceinline__ void split_sw_ref(const Phys& ph, R g, R c, R d, R u, R v, R w, R A1, R A2, R A3, R* fp,
+                                             R* fm) {
   const R tmp1 = R(2) * (g - R(1));
+#if OCFD_FEWER_DIVS
+  const R tmp3 = R(ph.sw_tmp3);
+#else
   const R tmp3 = (R(3) - g) / (R(2) * (g - R(1)));
+#endif
+#if OCFD_FEWER_DIVS
+  const R s2 = A1 * A1 + A2 * A2 + A3 * A3;
+  R ss1 = rsqrt(s2);
+  R ss = s2 * ss1;
+#else
   R ss = sqrt(A1 * A1 + A2 * A2 + A3 * A3);
   R ss1 = R(1) / ss;
+#endif
   R ak1 = A1 * ss1, ak2 = A2 * ss1, ak3 = A3 * ss1;
   R vs = A1 * u + A2 * v + A3 * w;
   R E1 = vs, E2 = vs - c * ss, E3 = vs + c * ss;
   R E1P = (E1 + fabs(E1)) * R(0.5), E2P = (E2 + fabs(E2)) * R(0.5), E3P = (E3 + fabs(E3)) * R(0.5);
   R E1M = E1 - E1P, E2M = E2 - E2P, E3M = E3 - E3P;
+#if OCFD_FEWER_DIVS
+  R tmp0 = d * R(ph.inv_2g);
+#else
   R tmp0 = d / (R(2) * g);
+#endif
   R uc1 = u - c * ak1, uc2 = u + c * ak1;
   R vc1 = v - c * ak2, vc2 = v + c * ak2;
   R wc1 = w - c * ak3, wc2 = w + c * ak3;
@@ -295,10 +315,15 @@ __device__ __forceinline__ void split_sw(const Phys& ph, R g, R c, R d, R u, R v
 // Local Lax-Friedrichs splitting of one point (eigenvalue bound per point):
 // split_Local_LaxFriedrichs, OCFD_flux_split.f90:73-104.
 template <typename R>
-__device__ __forceinline__ void split_llf(const Phys& ph, R g, R c, R d, R u, R v, R w, R A1, R A2, R A3, R* fp,
-                                          R* fm) {
+__device__ __forceinline__ void split_llf_ref(const Phys& ph, R g, R c, R d, R u, R v, R w, R A1, R A2, R A3, R* fp,
+                                              R* fm) {
+#if OCFD_FEWER_DIVS
+  const R tmp0 = R(ph.inv_g);
+  const R tmp1 = R(ph.inv_gm1);
+#else
   const R tmp0 = R(1) / g;
   const R tmp1 = R(1) / (g - R(1));
+#endif
   R ss = sqrt(A1 * A1 + A2 * A2 + A3 * A3);
   R un = A1 * u + A2 * v + A3 * w;
   R lamda0 = fabs(un) + ss * c;
@@ -316,7 +341,71 @@ __device__ __forceinline__ void split_llf(const Phys& ph, R g, R c, R d, R u, R 
   fm[3] = R(0.5) * (d * w * un + A3 * p1 - lamda0 * d * w);
   fm[4] = R(0.5) * (h0 * un - lamda0 * E0);
 }
-#endif
+
+// The splittings for a sweep whose metric row has a single non-zero component,
+// the one along the sweep (box and 1-D grids; production build only): A is
+// that component, |grad xi| = |A| and the unit normal is sign(A) along DIR, so
+// the square root, the reciprocal and the products with the zero components of
+// the general forms above drop out (results move by rounding only).
+template <int DIR, typename R>
+__device__ __forceinline__ void split_sw_axis_ref(const Phys& ph, R g, R c, R d, R u, R v, R w, R A, R* fp, R* fm) {
+  const R tmp1 = R(2) * (g - R(1));
+  const R tmp3 = R(ph.sw_tmp3);
+  const R ss = fabs(A);
+  const R cs = c * copysign(R(1), A);  // c ak_DIR
+  const R vs = A * (DIR == 0 ? u : (DIR == 1 ? v : w));
+  R E1 = vs, E2 = vs - c * ss, E3 = vs + c * ss;
+  R E1P = (E1 + fabs(E1)) * R(0.5), E2P = (E2 + fabs(E2)) * R(0.5), E3P = (E3 + fabs(E3)) * R(0.5);
+  R E1M = E1 - E1P, E2M = E2 - E2P, E3M = E3 - E3P;
+  R tmp0 = d * R(ph.inv_2g);
+  R uc1 = u, uc2 = u, vc1 = v, vc2 = v, wc1 = w, wc2 = w;
+  if (DIR == 0) {
+    uc1 = u - cs;
+    uc2 = u + cs;
+  } else if (DIR == 1) {
+    vc1 = v - cs;
+    vc2 = v + cs;
+  } else {
+    wc1 = w - cs;
+    wc2 = w + cs;
+  }
+  R vvc1 = (uc1 * uc1 + vc1 * vc1 + wc1 * wc1) * R(0.5);
+  R vvc2 = (uc2 * uc2 + vc2 * vc2 + wc2 * wc2) * R(0.5);
+  R vv = (g - R(1)) * (u * u + v * v + w * w);
+  R W2 = tmp3 * c * c;
+  fp[0] = tmp0 * (tmp1 * E1P + E2P + E3P);
+  fp[1] = tmp0 * (tmp1 * E1P * u + E2P * uc1 + E3P * uc2);
+  fp[2] = tmp0 * (tmp1 * E1P * v + E2P * vc1 + E3P * vc2);
+  fp[3] = tmp0 * (tmp1 * E1P * w + E2P * wc1 + E3P * wc2);
+  fp[4] = tmp0 * (E1P * vv + E2P * vvc1 + E3P * vvc2 + W2 * (E2P + E3P));
+  fm[0] = tmp0 * (tmp1 * E1M + E2M + E3M);
+  fm[1] = tmp0 * (tmp1 * E1M * u + E2M * uc1 + E3M * uc2);
+  fm[2] = tmp0 * (tmp1 * E1M * v + E2M * vc1 + E3M * vc2);
+  fm[3] = tmp0 * (tmp1 * E1M * w + E2M * wc1 + E3M * wc2);
+  fm[4] = tmp0 * (E1M * vv + E2M * vvc1 + E3M * vvc2 + W2 * (E2M + E3M));
+}
+
+template <int DIR, typename R>
+__device__ __forceinline__ void split_llf_axis_ref(const Phys& ph, R g, R c, R d, R u, R v, R w, R A, R* fp, R* fm) {
+  const R tmp0 = R(ph.inv_g);
+  const R tmp1 = R(ph.inv_gm1);
+  const R un = A * (DIR == 0 ? u : (DIR == 1 ? v : w));
+  const R lamda0 = fabs(un) + fabs(A) * c;
+  const R p1 = tmp0 * d * c * c;
+  const R E0 = tmp1 * p1 + R(0.5) * d * (u * u + v * v + w * w);
+  const R h0 = E0 + p1;
+  const R Ap = A * p1;
+  fp[0] = R(0.5) * (d * un + lamda0 * d);
+  fp[1] = R(0.5) * (DIR == 0 ? d * u * un + Ap + lamda0 * d * u : d * u * un + lamda0 * d * u);
+  fp[2] = R(0.5) * (DIR == 1 ? d * v * un + Ap + lamda0 * d * v : d * v * un + lamda0 * d * v);
+  fp[3] = R(0.5) * (DIR == 2 ? d * w * un + Ap + lamda0 * d * w : d * w * un + lamda0 * d * w);
+  fp[4] = R(0.5) * (h0 * un + lamda0 * E0);
+  fm[0] = R(0.5) * (d * un - lamda0 * d);
+  fm[1] = R(0.5) * (DIR == 0 ? d * u * un + Ap - lamda0 * d * u : d * u * un - lamda0 * d * u);
+  fm[2] = R(0.5) * (DIR == 1 ? d * v * un + Ap - lamda0 * d * v : d * v * un - lamda0 * d * v);
+  fm[3] = R(0.5) * (DIR == 2 ? d * w * un + Ap - lamda0 * d * w : d * w * un - lamda0 * d * w);
+  fm[4] = R(0.5) * (h0 * un - lamda0 * E0);
+}
 
 // Metric row of sweep DIR (A?1 arrays 13 + 3 DIR .. 15 + 3 DIR) has its two
 // off-diagonal components identically +0.0.

@@ -30,7 +30,7 @@ namespace ocfd {
 // Tile shapes (NP pencils x TF faces, one face per thread).  Variants 0 and 1
 // (256 threads) are the choices of the batch autotuner -- variant 1 (TF = 32)
 // wastes fewer threads on short pencils.  Variant 2 (128 threads) is the
-// single-instance tile of the characteristic OMP6 and the hybrid sweeps: at 256^3
+// single-instance tile of the characteristic OMP6 and the FP64 hybrid sweeps: at 256^3
 // it measured 5-9% faster with OMP6 than variant 0 (four blocks per SM overlap one
 // another's barrier and load phases better than two), but slower on the WENO7
 // sweeps, which keep variant 0.  Variants 3 (64 threads) and 4 (128
@@ -104,8 +104,8 @@ struct FaceTileV<2, 4> {
 // more to the halved number of threads (a step at 256^3 14.12 -> 14.31 ms).
 template <int DIR, bool CHAR, int SCHEME, typename R, bool ALLIN>
 struct FaceTile {
-  static constexpr bool HYB = OCFD_FEWER_DIVS && SCHEME == SCH_HYBRID;
-  static constexpr int FPT = (HYB && ALLIN && sizeof(R) == 8) ? 2 : 1;
+  static constexpr bool HYB = OCFD_FEWER_DIVS && SCHEME == SCH_HYBRID && sizeof(R) == 8;
+  static constexpr int FPT = HYB && ALLIN ? 2 : 1;
   using V = FaceTileV<DIR, ((CHAR && SCHEME == SCH_OMP6) || HYB) ? 2 : 0>;
   static constexpr int NP = FPT > 1 ? 8 : V::NP, TF = FPT > 1 ? 32 : V::TF, NT = NP * TF / FPT;
 };
@@ -290,6 +290,13 @@ constexpr int face_ps() {
   return (CHAR && sizeof(R) == 4 && DIR != 2) ? 20 : 1;
 }
 
+// The mixed-precision hybrid: FP32 sweeps with the reference's splitting sums and
+// schemes on stencil values (ocfd_face_values.cuh gives the reason).
+template <int SCHEME, typename R>
+constexpr bool face_on_values() {
+  return OCFD_FEWER_DIVS && SCHEME == SCH_HYBRID && sizeof(R) == 4;
+}
+
 // Block-wide list of the faces that leave a sweep's common path (production
 // build): the hybrid scheme's WENO faces, and in the characteristic form of a
 // non-periodic direction the faces of the boundary closures.  Where the sensor is
@@ -310,8 +317,9 @@ struct FaceList {
     return ((size_t)NVAL * sizeof(R) + NF * sizeof(unsigned short) + 15) / 16 * 16;
   }
 };
-template <bool CHAR, int SCHEME, bool ALLIN>
+template <bool CHAR, int SCHEME, bool ALLIN, typename R>
 constexpr bool face_has_list() {
+  if (face_on_values<SCHEME, R>()) return !CHAR;
   return OCFD_FEWER_DIVS && (SCHEME == SCH_HYBRID || (CHAR && !ALLIN));
 }
 template <bool CHAR, int SCHEME>
@@ -343,10 +351,16 @@ struct LimQueue {
 // bytes of a sweep's queues in shared memory: limiter queue, face list, three counts
 template <bool CHAR, int SCHEME, bool ALLIN, int NF, typename R>
 constexpr size_t face_queue() {
-  constexpr bool lim = face_has_limiter<CHAR, SCHEME>(), list = face_has_list<CHAR, SCHEME, ALLIN>();
+  constexpr bool lim = face_has_limiter<CHAR, SCHEME>(), list = face_has_list<CHAR, SCHEME, ALLIN, R>();
   return (lim ? LimQueue<NF>::template bytes<R>() : 0) + (list ? FaceList<NF, CHAR>::template bytes<R>() : 0) +
          (lim || list ? 16 : 0);
 }
+
+}  // namespace ocfd
+
+#include "ocfd_face_values.cuh"
+
+namespace ocfd {
 
 // Characteristic basis of one face, production build: the rows of L = S and
 // R = S^-1 of flux_charteric (OCFD_inviscous_character.f90:216-248) applied
@@ -587,11 +601,10 @@ __device__ __forceinline__ R lim_eval(const W& win, int r, int minus, R p0, R gm
 // non-zero component (axis_aligned); the splitting and the characteristic
 // basis use the axis-aligned forms.
 // FPT > 1: that many consecutive faces a thread (NP * TF / FPT threads).
-template <int DIR, bool CHAR, int SCHEME, bool ALLIN, int NP, int TF, typename R, typename S, bool TMA = false,
-          bool AXS = false, int FPT = 1>
-__device__ __forceinline__ void face_body(const FaceArgs<S>& a, const int bx, const int by, const int bz, R* sm,
-                                          const S* tile = nullptr, int toff = 0, R* qbase = nullptr,
-                                          int* qcount = nullptr) {
+template <int DIR, bool CHAR, int SCHEME, bool ALLIN, int NP, int TF, typename R, typename S, bool TMA, bool AXS,
+          int FPT>
+__device__ __forceinline__ void face_body_main(const FaceArgs<S>& a, const int bx, const int by, const int bz, R* sm,
+                                               const S* tile, int toff, R* qbase, int* qcount) {
   constexpr int LT = TF + 7;
   // shared memory (face_ps).  Records (PS > 1): F+ and F- each start on a
   // 16-byte boundary (GAP unused values after F+), so that four components of
@@ -648,7 +661,7 @@ __device__ __forceinline__ void face_body(const FaceArgs<S>& a, const int bx, co
   // with the staged input tile, dead after phase 1; the counts, written before
   // phase 1, then lie past that tile, at qcount).  Deferred OMP6 limiter: JC values,
   // JC tags (face of the tile * 16 + component * 2 + side); face list: values, faces.
-  constexpr bool DEFER = face_has_limiter<CHAR, SCHEME>(), LIST = face_has_list<CHAR, SCHEME, ALLIN>();
+  constexpr bool DEFER = face_has_limiter<CHAR, SCHEME>(), LIST = face_has_list<CHAR, SCHEME, ALLIN, R>();
   constexpr bool HQ = SCHEME == SCH_HYBRID && OCFD_FEWER_DIVS;
   // WENO sweeps of the production build work on stencil differences
   constexpr bool WDIFF = (SCHEME == SCH_WENO5 || SCHEME == SCH_WENO7) && OCFD_FEWER_DIVS;
@@ -747,14 +760,18 @@ __device__ __forceinline__ void face_body(const FaceArgs<S>& a, const int bx, co
         split_sw_axis<DIR>(ph, gam, c, d, u, v, w, Ad, fp, fm);
       else
         split_llf_axis<DIR>(ph, gam, c, d, u, v, w, Ad, fp, fm);
-    } else
-#endif
-    {
+    } else {
       if (a.split == 1)
         split_sw(ph, gam, c, d, u, v, w, A1, A2, A3, fp, fm);
       else
         split_llf(ph, gam, c, d, u, v, w, A1, A2, A3, fp, fm);
     }
+#else
+    if (a.split == 1)
+      split_sw_ref(ph, gam, c, d, u, v, w, A1, A2, A3, fp, fm);
+    else
+      split_llf_ref(ph, gam, c, d, u, v, w, A1, A2, A3, fp, fm);
+#endif
     if constexpr (PS > 1) {
       // the point's record in 16-byte stores (the unused slots get zeros)
       float4* r4 = reinterpret_cast<float4*>(sm + PI(l, p) * PS);
@@ -1555,14 +1572,29 @@ __device__ __forceinline__ void face_body(const FaceArgs<S>& a, const int bx, co
   }
 }
 
-template <int DIR, bool CHAR, int NP, int TF, typename R, bool AXS = false, int FPT = 1>
+// The body of every sweep: the mixed-precision hybrid keeps its own arithmetic
+// (ocfd_face_values.cuh).
+template <int DIR, bool CHAR, int SCHEME, bool ALLIN, int NP, int TF, typename R, typename S, bool TMA = false,
+          bool AXS = false, int FPT = 1>
+__device__ __forceinline__ void face_body(const FaceArgs<S>& a, const int bx, const int by, const int bz, R* sm,
+                                          const S* tile = nullptr, int toff = 0, R* qbase = nullptr,
+                                          int* qcount = nullptr) {
+  if constexpr (face_on_values<SCHEME, R>())
+    face_body_values<DIR, CHAR, ALLIN, NP, TF, R, S, TMA, AXS>(a, bx, by, bz, sm, tile, toff, qbase, qcount);
+  else
+    face_body_main<DIR, CHAR, SCHEME, ALLIN, NP, TF, R, S, TMA, AXS, FPT>(a, bx, by, bz, sm, tile, toff, qbase,
+                                                                         qcount);
+}
+
+template <int DIR, bool CHAR, int SCHEME, int NP, int TF, typename R, bool AXS = false, int FPT = 1>
 constexpr size_t face_smem_points() {
-  return (size_t)face_nvar<CHAR, AXS, (FPT > 1 ? 1 : face_ps<DIR, CHAR, R>())>() * face_points<FPT, NP, TF>() *
+  constexpr bool ax = AXS && !face_on_values<SCHEME, R>();
+  return (size_t)face_nvar<CHAR, ax, (FPT > 1 ? 1 : face_ps<DIR, CHAR, R>())>() * face_points<FPT, NP, TF>() *
          sizeof(R);
 }
 template <int DIR, bool CHAR, int SCHEME, int NP, int TF, typename R, bool AXS = false, int FPT = 1, bool ALLIN = true>
 constexpr size_t face_smem() {
-  return face_smem_points<DIR, CHAR, NP, TF, R, AXS, FPT>() + face_queue<CHAR, SCHEME, ALLIN, NP * TF, R>();
+  return face_smem_points<DIR, CHAR, SCHEME, NP, TF, R, AXS, FPT>() + face_queue<CHAR, SCHEME, ALLIN, NP * TF, R>();
 }
 // TMA sweeps: the queue shares memory with the staged input tiles
 // (read only in phase 1, the queue is used after phase 1's barrier); its entry
@@ -1576,7 +1608,7 @@ struct FaceTmaSmem {
   static constexpr bool QUEUE = QB != 0;
   static constexpr size_t COUNT_AT = TILE > QB ? TILE : QB;
   static constexpr size_t UNION = QUEUE ? COUNT_AT + 128 : TILE;  // before the staged points
-  static constexpr size_t BYTES = 128 + UNION + face_smem_points<DIR, CHAR, NP, TF, R, AXS, FPT>();
+  static constexpr size_t BYTES = 128 + UNION + face_smem_points<DIR, CHAR, SCHEME, NP, TF, R, AXS, FPT>();
 };
 
 // Minimum resident blocks per SM.  FP64: two (<= 128 registers) measured
