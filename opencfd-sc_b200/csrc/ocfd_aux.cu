@@ -71,18 +71,21 @@ __device__ __forceinline__ void decode(const Grid& G, long long t, int& i, int& 
   k = (int)(t / ((long long)G.nx * G.ny)) + 1;
 }
 
-// f(i, j, k) at every interior point: the blocks stride over 32 x 8 tiles of the
-// planes (256 threads), so that a point's indices cost no division; decoding a
-// linear index takes three 64-bit ones, which were half of the time of the
-// diagnostics (192^3: ana_box, Q and show_flow_msg, with the download of Q, 2.38 -> 1.92 ms).
+// f(i, j, k) at every interior point: the blocks (256 threads) stride over runs of 256
+// points of the planes, so that a point's indices cost one 32-bit division; decoding a
+// linear index takes three 64-bit ones.  us, decoded / so: show_flow_msg 192^3 157 / 149,
+// 8x400x300 50 / 49; ana_box 192^3 609 / 442, 8x400x300 160 / 122, 33x160x200 140 / 112.
+// (Tiles of 32 x 8 points need no division, but a row that fills them badly costs more:
+// 442 -> 456 at 192^3, 122 -> 259 at 8x400x300, 112 -> 161 at 33x160x200.)
 template <typename F>
 __device__ __forceinline__ void for_points(const Grid& G, F f) {
-  const int gx = (G.nx + 31) / 32, gy = (G.ny + 7) / 8, tiles = gx * gy * G.nz;
-  const int di = threadIdx.x & 31, dj = threadIdx.x >> 5;
-  for (int b = blockIdx.x; b < tiles; b += gridDim.x) {
-    const int r = b / gx, k = r / gy;
-    const int i = (b - r * gx) * 32 + di + 1, j = (r - k * gy) * 8 + dj + 1;
-    if (i <= G.nx && j <= G.ny) f(i, j, k + 1);
+  const unsigned nx = G.nx, plane = nx * (unsigned)G.ny;
+  const int runs = (int)((plane + 255) / 256);
+  const int total = runs * G.nz;
+  for (int b = blockIdx.x; b < total; b += gridDim.x) {
+    const int k = b / runs;
+    const unsigned p = (unsigned)(b - k * runs) * 256 + threadIdx.x, j = p / nx;
+    if (p < plane) f((int)(p - j * nx) + 1, (int)j + 1, k + 1);
   }
 }
 
@@ -692,44 +695,55 @@ cudaError_t launch_ana_box(const Grid& g, const Phys& ph, const DCoef& dc, doubl
 // Analysis of OCFD_analysis (OCFD_ANA.f90:3-31) beyond ana_box.
 
 // ana_getQ (OCFD_ANA.f90:127-171): Q = II(grad u) from the CD6/CD8 derivatives of
-// u, v, w (halos exchanged by the caller) and the metrics.
+// u, v, w (halos exchanged by the caller) and the metrics.  A block is a tile of
+// 32 x 8 points of a plane, or, for rows of less than 64, a run of 256 points of it: short
+// rows fill the tiles badly (us with the download, tiles / runs: 8x400x300 290 / 218,
+// 33x160x200 241 / 225, 65x130x130 235 / 233), long ones read the tile's neighbouring
+// rows from L1 (130^3 431 / 443, 192^3 1268 / 1346).
 __global__ void __launch_bounds__(256) k_ana_q(Grid G, Phys ph, DCoef dc, const double* u, const double* v,
-                                               const double* w, MetPtrs mp, double* q) {
+                                               const double* w, MetPtrs mp, double* q, bool tiled) {
   const int cd8 = ph.scheme_vis == 6;
   auto M = [&](int m, long long c) -> double { return met_at<double>(ph, m, mp.m[m], c); };
-  {
-    const int i = blockIdx.x * 32 + (threadIdx.x & 31) + 1;
-    const int j = blockIdx.y * 8 + (threadIdx.x >> 5) + 1;
-    const int k = blockIdx.z + 1;
-    if (i > G.nx || j > G.ny) return;
-    const long long c = G.ih(i, j, k);
-    const long long st[3] = {1, (long long)G.nxh, (long long)G.nxh * G.nyh};
-    const int l[3] = {i, j, k};
-    const double* q3[3] = {u, v, w};
-    double gr[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int dd = 0; dd < 3; dd++) gr[a][dd] = d0h(q3[a] + c, st[dd], l[dd], G.len(dd), ph.periodic[dd], cd8, dc, dd);
-    const double Akx = M(3, c), Aky = M(4, c), Akz = M(5, c), Aix = M(6, c), Aiy = M(7, c), Aiz = M(8, c);
-    const double Asx = M(9, c), Asy = M(10, c), Asz = M(11, c);
-    const double ux = gr[0][0] * Akx + gr[0][1] * Aix + gr[0][2] * Asx;
-    const double vx = gr[1][0] * Akx + gr[1][1] * Aix + gr[1][2] * Asx;
-    const double wx = gr[2][0] * Akx + gr[2][1] * Aix + gr[2][2] * Asx;
-    const double uy = gr[0][0] * Aky + gr[0][1] * Aiy + gr[0][2] * Asy;
-    const double vy = gr[1][0] * Aky + gr[1][1] * Aiy + gr[1][2] * Asy;
-    const double wy = gr[2][0] * Aky + gr[2][1] * Aiy + gr[2][2] * Asy;
-    const double uz = gr[0][0] * Akz + gr[0][1] * Aiz + gr[0][2] * Asz;
-    const double vz = gr[1][0] * Akz + gr[1][1] * Aiz + gr[1][2] * Asz;
-    const double wz = gr[2][0] * Akz + gr[2][1] * Aiz + gr[2][2] * Asz;
-    q[G.ii(i, j, k)] = ux * vy + ux * wz + vy * wz - uy * vx - uz * wx - vz * wy;
+  const int k = blockIdx.z + 1;
+  int i, j;
+  if (tiled) {
+    i = blockIdx.x * 32 + (threadIdx.x & 31) + 1;
+    j = blockIdx.y * 8 + (threadIdx.x >> 5) + 1;
+  } else {
+    const unsigned p = blockIdx.x * 256 + threadIdx.x, row = p / (unsigned)G.nx;
+    i = (int)(p - row * G.nx) + 1;
+    j = (int)row + 1;
   }
+  if (i > G.nx || j > G.ny) return;
+  const long long c = G.ih(i, j, k);
+  const long long st[3] = {1, (long long)G.nxh, (long long)G.nxh * G.nyh};
+  const int l[3] = {i, j, k};
+  const double* q3[3] = {u, v, w};
+  double gr[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int dd = 0; dd < 3; dd++) gr[a][dd] = d0h(q3[a] + c, st[dd], l[dd], G.len(dd), ph.periodic[dd], cd8, dc, dd);
+  const double Akx = M(3, c), Aky = M(4, c), Akz = M(5, c), Aix = M(6, c), Aiy = M(7, c), Aiz = M(8, c);
+  const double Asx = M(9, c), Asy = M(10, c), Asz = M(11, c);
+  const double ux = gr[0][0] * Akx + gr[0][1] * Aix + gr[0][2] * Asx;
+  const double vx = gr[1][0] * Akx + gr[1][1] * Aix + gr[1][2] * Asx;
+  const double wx = gr[2][0] * Akx + gr[2][1] * Aix + gr[2][2] * Asx;
+  const double uy = gr[0][0] * Aky + gr[0][1] * Aiy + gr[0][2] * Asy;
+  const double vy = gr[1][0] * Aky + gr[1][1] * Aiy + gr[1][2] * Asy;
+  const double wy = gr[2][0] * Aky + gr[2][1] * Aiy + gr[2][2] * Asy;
+  const double uz = gr[0][0] * Akz + gr[0][1] * Aiz + gr[0][2] * Asz;
+  const double vz = gr[1][0] * Akz + gr[1][1] * Aiz + gr[1][2] * Asz;
+  const double wz = gr[2][0] * Akz + gr[2][1] * Aiz + gr[2][2] * Asz;
+  q[G.ii(i, j, k)] = ux * vy + ux * wz + vy * wz - uy * vx - uz * wx - vz * wy;
 }
 cudaError_t launch_ana_q(const Grid& g, const Phys& ph, const DCoef& dc, double* const prim[5],
                          const double* const met[22], double* q, cudaStream_t st) {
   MetPtrs mp;
   for (int m = 0; m < 22; m++) mp.m[m] = const_cast<double*>(met[m]);
-  k_ana_q<<<update_dims(g), 256, 0, st>>>(g, ph, dc, prim[1], prim[2], prim[3], mp, q);
+  const bool tiled = g.nx >= 64;
+  const dim3 grid = tiled ? update_dims(g) : dim3(((unsigned)g.nx * g.ny + 255) / 256, 1, g.nz);
+  k_ana_q<<<grid, 256, 0, st>>>(g, ph, dc, prim[1], prim[2], prim[3], mp, q, tiled);
   return cudaGetLastError();
 }
 
@@ -738,11 +752,12 @@ cudaError_t launch_ana_q(const Grid& g, const Phys& ph, const DCoef& dc, double*
 __global__ void k_ana_average(Grid G, const double* d, const double* u, const double* v, const double* w,
                               const double* T, double* mean, double K) {
   const double* Q[5] = {d, u, v, w, T};
-  for_points(G, [&](int i, int j, int k) {
-    const long long c = G.ih(i, j, k), t = G.ii(i, j, k);
-#pragma unroll
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < G.n; t += (long long)gridDim.x * blockDim.x) {
+    int i, j, k;
+    decode(G, t, i, j, k);
+    const long long c = G.ih(i, j, k);
     for (int a = 0; a < 5; a++) mean[t + a * G.n] = (K * mean[t + a * G.n] + Q[a][c]) / (K + 1.0);
-  });
+  }
 }
 cudaError_t launch_ana_average(const Grid& g, double* const prim[5], double* mean, int K, cudaStream_t st) {
   k_ana_average<<<148 * 8, 256, 0, st>>>(g, prim[0], prim[1], prim[2], prim[3], prim[4], mean, (double)K);

@@ -1,4 +1,5 @@
-"""Diagnostics whose blocks walk 32 x 8 tiles: planes narrower than a tile, tiles cut in
+"""Diagnostics whose blocks walk runs of 256 points of a plane (Q in rows of 64 and more:
+tiles of 32 x 8): planes smaller than a run, runs and tiles cut in
 each direction, more tiles than blocks, box and body-fitted grids.  Q and the time
 averages are point by point (the strict build gives the oracle's bits); the sums of
 show_flow_msg and ana_box are taken in another order: n eps bounds the difference of two
@@ -16,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("strict", [True, False], ids=["strict", "fast"])
-@pytest.mark.parametrize("n", [(8, 8, 9), (33, 9, 10), (31, 23, 8), (64, 40, 57)], ids=lambda n: "x".join(map(str, n)))
+@pytest.mark.parametrize("n", [(8, 8, 9), (33, 9, 10), (31, 23, 8), (64, 40, 57), (8, 37, 60), (13, 35, 40)], ids=lambda n: "x".join(map(str, n)))
 @pytest.mark.parametrize("box", [True, False], ids=["box", "curvilinear"])
 def test_diagnostics(box, n, strict):
     if not box:  # the boundary closures need more points than the smallest box
