@@ -305,8 +305,8 @@ constexpr bool face_on_values() {
 // hold up every warp that meets one.  So the common faces are finished at once,
 // the others listed in shared memory (WENO7 faces from the front, the rest from
 // the back), and the block evaluates (face, component) pairs one a thread,
-// neighbouring threads on one component of neighbouring entries.  A tile in which
-// every face is listed does the work it did before.  The characteristic form keeps
+// neighbouring threads on one component of neighbouring entries (long lists of hybrid
+// faces: on two or three).  The characteristic form keeps
 // the five values of a face (the change relative to its upwind points) for the
 // face's own thread to project back.
 template <int NF, bool CHAR>
@@ -1470,7 +1470,60 @@ __device__ __forceinline__ void face_body_main(const FaceArgs<S>& a, const int b
     __syncthreads();
     const int n7 = ln[0], nj = n7 + ln[1];
     const R gm1 = xadd(R(ph.gamma), R(-1));
-    for (int e = threadIdx.x; e < 5 * nj; e += NT) {
+    // Hybrid faces of the characteristic form.  A list longer than one round of one-row
+    // items: an item is rows 0, 3, 4 or rows 1, 2 of a face, because one row an item reads
+    // the window five times and a tile with many WENO faces is then bound by shared memory.
+    // The three sweeps of 128x120x112 in ms per step, one row an item / grouped: noise
+    // everywhere (every face listed) 3.17 / 2.04, noise at 3% of the points 1.19 / 1.10; a
+    // short list has too few grouped items (noise at 1%: 0.86 / 0.93).
+    constexpr bool GROUPS = CHAR && HQ && ALLIN;
+    const bool group = GROUPS && 5 * nj > NT;
+    if (GROUPS && group) {
+      for (int e = threadIdx.x; e < 2 * nj; e += NT) {
+        const bool lm = e >= nj;  // rows 1, 2
+        const int x = lm ? e - nj : e, slot = x < n7 ? x : NP * TF - 1 - (x - n7);
+        const auto win = window(ltag[slot]);
+        auto mean = [&](int var) -> R { return xmul(xadd(win(var, 3), win(var, 4)), R(0.5)); };
+        const int row[3] = {lm ? 1 : 0, lm ? 2 : 3, 4};
+        R L[3][5];
+        {
+          CharBasis<DIR, AXS, R> cb;
+          cb.init(mean(10), mean(11), mean(12), mean(13), AXS ? R(0) : mean(14), AXS ? R(0) : mean(15),
+                  AXS ? R(0) : mean(16));
+          const R rc = xrcp(cb.c), KK = xmul(gm1, xmul(rc, rc)), X1 = xmul(R(0.5), rc), V2 = cb.V2();
+#pragma unroll
+          for (int r = 0; r < 3; r++) cb.row(row[r], KK, X1, V2, L[r]);
+        }
+        R h[3];
+#pragma unroll 1
+        for (int side = 0; side < 2; side++) {
+          R d[3][6], last[3];
+#pragma unroll
+          for (int k = 0; k < 7; k++) {  // F+ at offsets -3..3, F- mirrored (4..-2)
+            R f[5];
+#pragma unroll
+            for (int v = 0; v < 5; v++) f[v] = win(5 * side + v, side ? 7 - k : k);
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+              const R y =
+                  xfma(L[r][4], f[4], xfma(L[r][3], f[3], xfma(L[r][2], f[2], xfma(L[r][1], f[1], xmul(L[r][0], f[0])))));
+              if (k > 0) d[r][k - 1] = xsub(y, last[r]);
+              last[r] = y;
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < 3; r++) {
+            if (r == 2 && lm) break;
+            const R y = x < n7 ? weno_diff<SCH_WENO7>(d[r]) : weno_diff<SCH_WENO5>(d[r]);
+            h[r] = side ? xadd(h[r], y) : y;
+          }
+        }
+        lv[row[0] * NP * TF + slot] = h[0];
+        lv[row[1] * NP * TF + slot] = h[1];
+        if (!lm) lv[4 * NP * TF + slot] = h[2];
+      }
+    }
+    for (int e = threadIdx.x; !group && e < 5 * nj; e += NT) {
       const int m = e / nj, x = e - m * nj;
       const int slot = x < n7 ? x : NP * TF - 1 - (x - n7);
       const int t = ltag[slot];
@@ -1636,7 +1689,9 @@ struct FaceTmaSmem {
 // threads and minimum resident blocks of the single-instance sweeps
 #define OCFD_FACE_NT (FaceTile<DIR, CHAR, SCHEME, R, ALLIN>::NT)
 #ifndef OCFD_FACE64_MINBPAIR
-#define OCFD_FACE64_MINBPAIR 5  // FP64, two faces a thread: 5 blocks of 128 (four: 0.5% slower)
+#define OCFD_FACE64_MINBPAIR (CHAR ? 4 : 5)  // FP64, two faces a thread: blocks of 128.  Flux-vector
+                                            // form 5 (four: 0.5% slower); the shared memory of
+                                            // the characteristic form allows four
 #endif
 #ifndef OCFD_FACE64_MINB128
 #define OCFD_FACE64_MINB128 4  // FP64, 128-thread tiles: 4 blocks (128 registers); 5 (96
