@@ -1041,6 +1041,7 @@ static void prof_mark(ocfd_handle* h, Prof* pf, int group) {
 // 0.987, mixed 0.508 / 0.518, 256^3 OMP6 14.1 / 16.7.
 constexpr long long PHASE_MAX_BYTES = 1LL << 20;
 static bool phase_merged(const ocfd_handle* h) {
+  if (h->mixed && face_tma32_enabled()) return false;  // FP32 TMA staging was asked for: the sweeps that have it
   return h->p.if_viscous && phase_supported(h->ph) && h->g.n * (h->mixed ? 4 : 8) <= PHASE_MAX_BYTES;
 }
 

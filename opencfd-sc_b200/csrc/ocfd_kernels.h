@@ -168,6 +168,7 @@ cudaError_t launch_visc_grad(const ViscArgs<R, S>& a, cudaStream_t st);
 template <typename R>
 cudaError_t launch_phase(bool chr, int scheme, const FaceArgs<R> f[3], const ViscArgs<R, R>& v, cudaStream_t st);
 cudaError_t setup_phase_kernels();
+bool face_tma32_enabled();  // OCFD_FACE_TMA32=1
 inline bool phase_supported(const Phys& ph) {
   return OCFD_FEWER_DIVS && ph.periodic[0] && ph.periodic[1] && ph.periodic[2] && axis_aligned<0>(ph.metzero) &&
          axis_aligned<1>(ph.metzero) && axis_aligned<2>(ph.metzero) && metrics_diagonal(ph.metzero);
