@@ -287,11 +287,18 @@ def test_mixed_precision_close_to_fp64():
     assert abs(eb[1] - ea[1]) / ea[1] < 1e-6
 
 
-@pytest.mark.parametrize("case", ["omp6char-fp64", "omp6char-mixed", "curvilinear-fp64"])
+@pytest.mark.parametrize("case", ["omp6char-fp64", "omp6char-mixed", "curvilinear-fp64", "hybrid-fp64", "hybrid-mixed",
+                                  "hybridchar-fp64", "hybridchar-mixed"])
 def test_same_bits_twice(case):
-    """Race check: the same run twice gives the same bits (the limiter queue's
-    entry order depends on atomics, its results must not)."""
-    if case.startswith("omp6char"):
+    """Race check: the same run twice gives the same bits (the entry order of the
+    limiter queue and of the face list depends on atomics, their results must not)."""
+    if case.startswith("hybrid"):
+        char = case.startswith("hybridchar")
+        p, X, prims = tgv_case(scheme=SCHEME_HYBRID, character=int(char), split=SPLIT_SW if char else SPLIT_LLF, ma=0.5,
+                               mixed=case.endswith("mixed"), n=(65, 40, 33))
+        rng = np.random.default_rng(17)  # WENO faces here and there, and in every face of one part
+        prims = [a * (1.0 + 1e-2 * rng.random(a.shape) * (np.arange(65) < 30)) for a in prims]
+    elif case.startswith("omp6char"):
         p, X, prims = tgv_case(scheme=SCHEME_OMP6, character=1, mixed=case.endswith("mixed"), n=(32, 24, 16))
     else:
         p, X, prims = curvilinear_case()
