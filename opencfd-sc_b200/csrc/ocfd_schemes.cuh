@@ -343,23 +343,23 @@ __device__ __forceinline__ T weno_diff(const T* e) {
 }
 // Sum of both sides' WENO values relative to their upwind points.  vp[k] = F+(k - 3),
 // vm[k] = F-(4 - k) (mirrored), k = 0..6; FP32: the sides in the two lanes.
-template <int SCHEME>
-__device__ __forceinline__ double weno_pair(const double* vp, const double* vm) {
-  double e[6];
+template <int SCHEME, typename R>
+__device__ __forceinline__ R weno_pair(const R* vp, const R* vm) {
+  if constexpr (OCFD_F32X2 && sizeof(R) == 4) {
+    F2 e[6];
 #pragma unroll
-  for (int k = 0; k < 6; k++) e[k] = xsub(vp[k + 1], vp[k]);
-  const double hp = weno_diff<SCHEME>(e);
+    for (int k = 0; k < 6; k++) e[k] = xsub(f2(vp[k + 1], vm[k + 1]), f2(vp[k], vm[k]));
+    const F2 h = weno_diff<SCHEME>(e);
+    return xadd(R(h.v.x), R(h.v.y));
+  } else {  // one side after the other, the same bits
+    R e[6];
 #pragma unroll
-  for (int k = 0; k < 6; k++) e[k] = xsub(vm[k + 1], vm[k]);
-  return xadd(hp, weno_diff<SCHEME>(e));
-}
-template <int SCHEME>
-__device__ __forceinline__ float weno_pair(const float* vp, const float* vm) {
-  F2 e[6];
+    for (int k = 0; k < 6; k++) e[k] = xsub(vp[k + 1], vp[k]);
+    const R hp = weno_diff<SCHEME>(e);
 #pragma unroll
-  for (int k = 0; k < 6; k++) e[k] = xsub(f2(vp[k + 1], vm[k + 1]), f2(vp[k], vm[k]));
-  const F2 h = weno_diff<SCHEME>(e);
-  return xadd(h.v.x, h.v.y);
+    for (int k = 0; k < 6; k++) e[k] = xsub(vm[k + 1], vm[k]);
+    return xadd(hp, weno_diff<SCHEME>(e));
+  }
 }
 
 // minmod2 / minmod4: OCFD_Schemes.f90:274-289
