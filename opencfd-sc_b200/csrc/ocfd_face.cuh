@@ -30,11 +30,11 @@ namespace ocfd {
 // Tile shapes (NP pencils x TF faces, one face per thread).  Variants 0 and 1
 // (256 threads) are the choices of the batch autotuner -- variant 1 (TF = 32)
 // wastes fewer threads on short pencils.  Variant 2 (128 threads) is the
-// single-instance tile of the characteristic OMP6 and the FP64 hybrid sweeps: at 256^3
+// single-instance tile of the characteristic OMP6 and the hybrid sweeps: at 256^3
 // it measured 5-9% faster with OMP6 than variant 0 (four blocks per SM overlap one
 // another's barrier and load phases better than two), but slower on the WENO7
-// sweeps, which keep variant 0.  Variants 3 (64 threads) and 4 (128
-// threads, TF = 32 along y and z) measured slower.
+// sweeps, which keep variant 0.  (Tiles of 64 threads, or of 128 with TF = 32 along y and
+// z, measured slower.)
 template <int DIR, int V>
 struct FaceTileV;
 template <>
@@ -74,26 +74,6 @@ template <>
 struct FaceTileV<2, 2> {
   static constexpr int NP = 8, TF = 16;
 };
-template <>
-struct FaceTileV<0, 3> {
-  static constexpr int NP = 1, TF = 64;
-};
-template <>
-struct FaceTileV<1, 3> {
-  static constexpr int NP = 4, TF = 16;
-};
-template <>
-struct FaceTileV<2, 3> {
-  static constexpr int NP = 4, TF = 16;
-};
-template <>
-struct FaceTileV<1, 4> {
-  static constexpr int NP = 4, TF = 32;
-};
-template <>
-struct FaceTileV<2, 4> {
-  static constexpr int NP = 4, TF = 32;
-};
 // Tile of a single-instance sweep: NP pencils x TF faces, NT threads, each FPT
 // consecutive faces.  Two faces a thread: the FP64 hybrid sweeps of periodic
 // directions.  Their common face is the linear scheme, 80 multiply-adds on 80 values
@@ -104,8 +84,8 @@ struct FaceTileV<2, 4> {
 // more to the halved number of threads (a step at 256^3 14.12 -> 14.31 ms).
 template <int DIR, bool CHAR, int SCHEME, typename R, bool ALLIN>
 struct FaceTile {
-  static constexpr bool HYB = OCFD_FEWER_DIVS && SCHEME == SCH_HYBRID && sizeof(R) == 8;
-  static constexpr int FPT = HYB && ALLIN ? 2 : 1;
+  static constexpr bool HYB = OCFD_FEWER_DIVS && SCHEME == SCH_HYBRID;
+  static constexpr int FPT = (HYB && ALLIN && sizeof(R) == 8) ? 2 : 1;
   using V = FaceTileV<DIR, ((CHAR && SCHEME == SCH_OMP6) || HYB) ? 2 : 0>;
   static constexpr int NP = FPT > 1 ? 8 : V::NP, TF = FPT > 1 ? 32 : V::TF, NT = NP * TF / FPT;
 };

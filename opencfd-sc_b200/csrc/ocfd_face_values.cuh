@@ -8,7 +8,7 @@
 // Lax-Friedrichs splitting, 25 steps: 3e-5 in the 2-norm between this arithmetic and
 // that of the differences, both within 6e-6 of the double-precision run).  Runs go on as
 // they were begun only if the arithmetic stays as it is, so it is kept here, at the price
-// of 10% of a step (192^3, ms per step: 3.31, on differences 3.01).  The splitting and the
+// of 5% of a step (192^3, ms per step: 3.18, on differences 3.03).  The splitting and the
 // schemes are plain sums that the compiler contracts, so a change of this file, or of how
 // it is inlined, is checked against stored digests (tests/test_gpu_mixed_hybrid.py).
 #pragma once
