@@ -572,7 +572,7 @@ def run_ours(args):
                                         "mode": "upload f + haloed primitives, one step, download both"}},
             "gpu_launches": launches,
             "roofline": {"bound": "hbm", "peak": peak, "unit": "GB/s", "peak_kind": peak_kind, **kern,
-                         "note": "the face kernels are FP64-pipe (FP64) or issue (FP32) bound, not HBM bound"},
+                         "note": "the face kernels are bound by shared memory, issue and latency, not by HBM"},
             "mixed": mixed,
             "served": served,
             "cpu_baseline": cpu,

@@ -299,7 +299,9 @@ int ocfd_gpu_step_kernels(const ocfd_handle* h);
  * group on the instance's stream; ms[] receives the average milliseconds per
  * step of: [0] shock sensor, [1] x faces, [2] y faces, [3] z faces, [4]
  * viscous gradients, [5] fused stage tail, [6] negative-T repair + BC +
- * halos, [7] the whole step.  Advances the solution like ocfd_gpu_step.
+ * halos, [7] the whole step.  Advances the solution like ocfd_gpu_step, to
+ * the same bits; on small grids, where ocfd_gpu_step runs the sweeps and the
+ * viscous gradients of a stage as one launch, they run and are timed as four.
  * (Timing instrumentation: the reference only times the whole loop with
  * MPI_wtime, OCFD_NS_Solver.f90:18-19,79-80.) */
 int ocfd_gpu_profile_steps(ocfd_handle* h, int nsteps, double ms[8]);

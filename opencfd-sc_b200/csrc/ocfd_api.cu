@@ -1032,13 +1032,19 @@ static void prof_mark(ocfd_handle* h, Prof* pf, int group) {
 }
 
 // The sweeps and the viscous gradients of a small grid go out as one launch
-// (ocfd_phase.cuh).  The line, 1 MiB an array (50^3 points in FP64, 64^3 in FP32), lies
-// where a sweep stops being about one wave of blocks, so that its launch gap and idle
-// SMs are most of its time.  Four launches against one, ms per step: WENO7 32^3 mixed
-// 0.064 / 0.047, FP64 0.092 / 0.069; hybrid 48^3 FP64 0.200 / 0.151; 64^3 mixed WENO7
-// 0.176 / 0.161, OMP6 0.213 / 0.186.  Past it the roles share one register and
-// shared-memory limit for nothing: 64^3 FP64 OMP6 0.326 / 0.348, 96^3 WENO7 0.951 /
-// 0.987, mixed 0.508 / 0.518, 256^3 OMP6 14.1 / 16.7.
+// (ocfd_phase.cuh), which fills the SMs that the last wave of each of four short launches
+// leaves idle and has one launch gap for four; on larger grids the roles share one register
+// and shared-memory limit for nothing.  The line, 1 MiB an array, lies at the last size at
+// which every scheme gains or is even.  ms per step, four launches / one, cubes:
+//   FP64    32            48            50            52            64
+//   WENO7   0.088/0.066   0.156/0.141   0.234/0.195   0.236/0.204   0.315/0.308
+//   OMP6 c  0.100/0.080   0.159/0.135   0.215/0.189   0.219/0.224   0.317/0.332
+//   hybr.c  0.085/0.069   0.126/0.124   0.177/0.179   0.182/0.198   0.257/0.279
+//   mixed   32            50            64            68            72
+//   WENO7   0.064/0.046   0.121/0.103   0.173/0.159   0.247/0.240   0.276/0.271
+//   WENO7 c 0.067/0.053   0.142/0.120   0.203/0.198   0.296/0.299   0.325/0.328
+//   OMP6 c  0.074/0.052   0.131/0.101   0.198/0.178   0.264/0.250   0.290/0.279
+//   hybrid  0.065/0.047   0.109/0.090   0.161/0.144   0.226/0.212   0.250/0.237
 constexpr long long PHASE_MAX_BYTES = 1LL << 20;
 static bool phase_merged(const ocfd_handle* h) {
   if (h->mixed && face_tma32_enabled()) return false;  // FP32 TMA staging was asked for: the sweeps that have it

@@ -36,10 +36,12 @@ bool face_tma_enabled() {
 }
 
 // TMA staging of the FP32 face sweeps: off unless OCFD_FACE_TMA32=1 (and the
-// driver offers a tensor-map encoder).  The FP32 sweeps compile to differently
-// contracted arithmetic in the TMA kernels than in the batched kernels (plain
-// loads), and a batched member must give the same bits as the same instance
-// stepped alone; the staged and the plain sweeps agree to FP32 rounding.
+// driver offers a tensor-map encoder), because plain loads are faster or equal on most
+// forms: ms per step, plain / TMA, OMP6 char 256^3 8.03 / 8.14, WENO7 char 192^3 4.27 / 4.32,
+// cylinder 301x401x8 1.18 / 1.18; flux-vector WENO7 256^3 8.28 / 8.22.  Both give the same
+// bits, but for the flux-vector hybrid, whose plain sums (ocfd_face_values.cuh) the compiler
+// contracts differently in the TMA kernels; a batched member, staged with plain loads, must
+// give the bits of the instance stepped alone.
 bool face_tma32_enabled() {
   static int on = -1;
   if (on < 0) {

@@ -4,7 +4,7 @@
 // The four are independent of one another: all read the primitives and the
 // metrics, each writes its own array.  A small grid's stage is bound by launch gaps
 // and by SMs without a block; one launch has one gap and one last wave instead of
-// four (WENO7 32^3 mixed 0.064 -> 0.047 ms per step; the line is in ocfd_api.cu).
+// four (WENO7 32^3 mixed 0.064 -> 0.046 ms per step; the line is in ocfd_api.cu).
 #pragma once
 
 #include "ocfd_face.cuh"
