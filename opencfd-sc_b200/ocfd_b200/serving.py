@@ -130,9 +130,11 @@ class Server:
         self.max_points = max_points
         # instances of at least solo_min^3 points advance on their own captured
         # step graphs (single-instance kernels, concurrently on their own
-        # streams): measured faster than their part of a batched launch; the
-        # smaller ones share the batched launches, which run several of them at
-        # once where alone each would leave most of the GPU idle
+        # streams): measured faster than their part of a batched launch (mixed
+        # WENO7, 2 x 96^3: 1.73 against 1.53 GPts/s); the smaller ones share the
+        # batched launches, which run several of them at once where alone each
+        # would leave most of the GPU idle (64 x 32^3: 0.69 against 1.36; at 48^3
+        # and 64^3 the two are within 3 and 9%, in favour of the instance alone)
         self.solo_min = solo_min
         # batched launch mode: "timed" (each new set of grid sizes times both modes
         # on its first round and keeps the faster), "per_kernel" or "persistent"
